@@ -1,0 +1,80 @@
+"""Traversal paths at the sizes where their dispatch changes: results against
+the CPU oracle (integers bit for bit)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _stars(gsrb, degrees, seed=1, whi=255):
+    """Hubs of the given degrees on a common pool of leaves, joined in a path."""
+    rng = np.random.default_rng(seed)
+    pool = max(degrees) + 16
+    src, dst = [], []
+    for i, d in enumerate(degrees):
+        leaves = rng.choice(pool, d - 1 - (0 < i < len(degrees) - 1), replace=False)  # path edges count too
+        src.append(np.full(leaves.size, pool + i))
+        dst.append(leaves)
+    k = len(degrees)
+    src.append(pool + np.arange(k - 1))
+    dst.append(pool + np.arange(1, k))
+    return gsrb.csr_from_edges(pool + k, np.concatenate(src), np.concatenate(dst), whi=whi), pool
+
+
+@pytest.fixture(scope="module")
+def path_graphs(gsrb):
+    rng = np.random.default_rng(3)
+    left, right = 2600, 300  # 2600 vertices of degree > 256: more hubs than one shared-memory list holds
+    bip = gsrb.csr_from_edges(left + right, np.repeat(np.arange(left), 260),
+                              left + np.concatenate([rng.choice(right, 260, replace=False) for _ in range(left)]))
+    return {
+        "degrees": _stars(gsrb, [255, 256, 257, 258, 31, 32, 33, 4095, 4096, 4097, 2])[0],
+        "bipartite": bip,
+        "grid": gsrb.grid2d(301, 77, seed=9),
+        "rmat": gsrb.rmat(13, 20, seed=5),
+    }
+
+
+@pytest.mark.parametrize("name", ["degrees", "bipartite", "grid", "rmat"])
+@pytest.mark.parametrize("shape", ["default", "one_cta", "three_ctas"])
+@pytest.mark.parametrize("delta", [3, 700, 1 << 30])
+def test_sssp_paths(gsrb, ctx, orc, path_graphs, name, shape, delta):
+    g = path_graphs[name]
+    dg = ctx.graph(g)
+    out = ctx.array(g.nnodes, np.int32)
+    c = None if shape == "default" else gsrb.cfg(variant=gsrb.BAR_FANOUT, threads=96,
+                                                 grid_override=1 if shape == "one_cta" else 3)
+    for src in (0, g.nnodes - 1):
+        rc, _ = dg.sssp(src, out, delta, c)
+        gsrb.check(rc, "sssp")
+        assert np.array_equal(out.download(), orc.dijkstra(g, src))
+
+
+def test_sssp_long_weights(gsrb, ctx, orc):
+    """Path lengths beyond INT_MAX are no paths (the sum saturates)."""
+    n = 12
+    g = gsrb.csr_from_edges(n, np.arange(n - 1), np.arange(1, n))
+    w = np.where(g.edge_data > 0, 2**29, 0).astype(np.int32)
+    g = gsrb.Graph(g.row_start, g.edge_dst, w)
+    dg = ctx.graph(g)
+    out = ctx.array(n, np.int32)
+    rc, _ = dg.sssp(0, out, 1 << 30)
+    gsrb.check(rc, "sssp")
+    want = [min(i * 2**29, 2**31 - 1) for i in range(4)] + [2**31 - 1] * (n - 4)
+    assert out.download().tolist() == want
+
+
+def test_batch_calls_back_to_back(gsrb, ctx, orc, path_graphs):
+    """Calls on one batch without a wait between them, each with other sources:
+    the last call's results stand."""
+    gs = [path_graphs["grid"], path_graphs["degrees"], path_graphs["rmat"]]
+    dgs = [ctx.graph(g) for g in gs]
+    outs = [[ctx.array(g.nnodes, np.int32) for g in gs] for _ in range(6)]
+    b = gsrb.Batch(ctx, dgs)
+    for i in range(6):
+        gsrb.check(b.sssp([i] * 3, outs[i], 500) if i % 2 else b.bfs([i] * 3, outs[i]), "batch")
+    rc, _ = b.stats()
+    gsrb.check(rc)
+    for i in range(6):
+        for g, o in zip(gs, outs[i]):
+            assert np.array_equal(o.download(), orc.dijkstra(g, i) if i % 2 else orc.bfs(g, i))

@@ -618,6 +618,13 @@ struct SsspArgs {
   unsigned long long* out_edges;
 };
 
+// Vertices of more edges than this go to the near hub queue and are relaxed
+// edge-balanced over the whole team, kHubList at a time (with 4096 and a list
+// per CTA above 256, R-MAT-17's second round waited for the CTAs whose share of
+// the frontier held the most edges: 93 -> 66 us).
+constexpr uint32_t kSsspBig = 256;
+constexpr uint32_t kProbeMeanDegree = 8;  // graphs of this mean degree probe before claiming in every round
+
 // Where an SSSP relax step puts the vertices whose distance it lowered.
 struct RelaxSink {
   uint32_t* qout;               // near queue of the next round
@@ -628,11 +635,19 @@ struct RelaxSink {
   unsigned long long* fc;
   uint32_t stamp;               // near-queue stamp of this round
   uint32_t fgen;                // far-pile generation
-  long long T;                  // near threshold
-  WarpRes* res;                 // the warp's near-queue reservation
+  int32_t T;                    // near threshold (at most kInf, which no queued distance reaches)
+  IdStage* stage;               // the CTA's near-queue entries
+  WarpRes* res;                 // the warp's near-queue reservation (past the stage)
   uint32_t near_cap;            // near-queue capacity in slots (holes included)
   bool precheck;                // read a distance before claiming it (large rounds)
 };
+
+// A path length at kInf or beyond is no path: the sum saturates there.
+__device__ __forceinline__ int32_t add_sat(int32_t a, int32_t b) {
+  int32_t r;
+  asm("add.sat.s32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 
 // Relax four edges per lane at once: edge r of the lane is j[r] (where bit r of
 // `act` is set), leaving a vertex at distance du[r].  Every dependent step is
@@ -644,48 +659,64 @@ struct RelaxSink {
 // whether the edge improves -- and the row range goes out with the claim.
 // The same claims land either way, so distances are the same.
 // Warp-synchronous.
-__device__ __forceinline__ void sssp_relax4e(const SsspArgs& a, const long long* du, const uint32_t* j, uint32_t act,
-                                             const RelaxSink& s, unsigned long long& my_edges) {
+__device__ __forceinline__ void sssp_relax4e(const SsspArgs& a, const int32_t* du, const uint32_t* j, uint32_t act,
+                                             const RelaxSink& s, uint32_t& my_edges) {
   const DevCSR& g = a.g;
   uint32_t v[4];
-  long long nd[4];
+  int32_t nd[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const bool on = (act >> r) & 1u;
     v[r] = on ? __ldg(g.dst + j[r]) : 0u;
-    nd[r] = on ? du[r] + (long long)__ldg(g.w + j[r]) : (long long)kInf;
-    my_edges += on ? 1u : 0u;
+    nd[r] = on ? add_sat(du[r], __ldg(g.w + j[r])) : kInf;
   }
+  my_edges += __popc(act);
+  // (Results of loads and atomics are only looked at in a loop of their own:
+  // a comparison inside the branch that issues an atomic would make the warp
+  // wait for each of the four in turn.)
   bool imp[4];
   uint32_t rb[4], re[4];
+  int32_t old[4];
   if (s.precheck) {
     int32_t cur[4];
 #pragma unroll
-    for (int r = 0; r < 4; ++r) cur[r] = nd[r] < (long long)kInf ? __ldcg(a.dist + v[r]) : kInf;
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-      imp[r] = nd[r] < (long long)cur[r] && nd[r] < (long long)atomicMin(a.dist + v[r], (int32_t)nd[r]);
-#pragma unroll
     for (int r = 0; r < 4; ++r) {
-      rb[r] = imp[r] && nd[r] < s.T ? __ldg(g.row + v[r]) : 0u;
-      re[r] = imp[r] && nd[r] < s.T ? __ldg(g.row + v[r] + 1) : 0u;
+      cur[r] = kInf;
+      if (nd[r] < kInf) cur[r] = __ldcg(a.dist + v[r]);
     }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) imp[r] = nd[r] < cur[r];
   } else {
 #pragma unroll
-    for (int r = 0; r < 4; ++r) {
-      const bool on = nd[r] < (long long)kInf;
-      rb[r] = on && nd[r] < s.T ? __ldg(g.row + v[r]) : 0u;
-      re[r] = on && nd[r] < s.T ? __ldg(g.row + v[r] + 1) : 0u;
-    }
+    for (int r = 0; r < 4; ++r) imp[r] = nd[r] < kInf;
+  }
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
-      imp[r] = nd[r] < (long long)kInf && nd[r] < (long long)atomicMin(a.dist + v[r], (int32_t)nd[r]);
+  for (int r = 0; r < 4; ++r) {
+    old[r] = 0;
+    if (imp[r]) old[r] = atomicMin(a.dist + v[r], nd[r]);
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    rb[r] = re[r] = 0;
+    if (imp[r] && nd[r] < s.T) {
+      rb[r] = __ldg(g.row + v[r]);
+      re[r] = __ldg(g.row + v[r] + 1);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) imp[r] = imp[r] && nd[r] < old[r];
+  uint32_t st[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    const bool near = nd[r] < s.T;
+    st[r] = 0;
+    if (imp[r]) st[r] = atomicExch((near ? a.mark : a.fmark) + v[r], near ? s.stamp : s.fgen);
   }
   bool to_near[4], to_far[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    to_near[r] = imp[r] && nd[r] < s.T && atomicExch(a.mark + v[r], s.stamp) != s.stamp;
-    to_far[r] = imp[r] && nd[r] >= s.T && atomicExch(a.fmark + v[r], s.fgen) != s.fgen;
+    to_near[r] = imp[r] && nd[r] < s.T && st[r] != s.stamp;
+    to_far[r] = imp[r] && nd[r] >= s.T && st[r] != s.fgen;
   }
   uint32_t d[4];
 #pragma unroll
@@ -693,28 +724,12 @@ __device__ __forceinline__ void sssp_relax4e(const SsspArgs& a, const long long*
   bool reg[4], big[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    reg[r] = to_near[r] && d[r] <= kBigDegree;
-    big[r] = to_near[r] && d[r] > kBigDegree;
+    reg[r] = to_near[r] && d[r] <= kSsspBig;
+    big[r] = to_near[r] && d[r] > kSsspBig;
   }
-  if (s.res->chunk) warp_append_res<4>(reg, v, s.qout, s.n_reg, s.near_cap, a.overflow, *s.res, kHole);
-  else warp_append_k<4>(reg, v, s.qout, s.n_reg, g.n, a.overflow);
+  stage_append<4>(reg, v, *s.stage, s.qout, s.n_reg, g.n, s.near_cap, a.overflow, *s.res, kHole);
   warp_append_k<4>(big, v, s.hout, s.n_big, g.n, a.overflow);
   warp_append_k<4>(to_far, v, s.fout, s.fc, g.n, a.overflow);
-}
-
-// The same from one vertex: edge r is jbase + r * stride while below jend.
-__device__ __forceinline__ void sssp_relax4(const SsspArgs& a, long long du, uint32_t jbase, uint32_t stride,
-                                            uint32_t jend, const RelaxSink& s, unsigned long long& my_edges) {
-  long long dd[4];
-  uint32_t j[4];
-  uint32_t act = 0;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    dd[r] = du;
-    j[r] = jbase + (uint32_t)r * stride;
-    if (j[r] < jend) act |= 1u << r;
-  }
-  sssp_relax4e(a, dd, j, act, s, my_edges);
 }
 
 // A list of vertices relaxed edge-balanced: their edge counts' prefix p[0..cnt]
@@ -723,10 +738,10 @@ __device__ __forceinline__ void sssp_relax4(const SsspArgs& a, long long du, uin
 // finding its vertex by binary search over p.  Warp-synchronous loops.
 __device__ __forceinline__ void sssp_relax_list(const SsspArgs& a, const uint32_t* p, const uint32_t* b,
                                                 const int32_t* d, uint32_t cnt, uint32_t x, uint32_t nthr,
-                                                const RelaxSink& s, unsigned long long& my_edges) {
+                                                const RelaxSink& s, uint32_t& my_edges) {
   const uint32_t total = p[cnt];
   for (uint32_t t0 = (x & ~31u) + lane_id(); t0 - lane_id() < total; t0 += 4u * nthr) {
-    long long du[4];
+    int32_t du[4];
     uint32_t j[4];
     uint32_t act = 0;
 #pragma unroll
@@ -745,18 +760,12 @@ __device__ __forceinline__ void sssp_relax_list(const SsspArgs& a, const uint32_
   }
 }
 
-// Vertices of the regular queue with more edges than this are relaxed by their
-// whole CTA (after the CTA's warps have walked their queue groups), so that one
-// warp does not walk thousands of edges while the rest of the grid waits at
-// the round's barrier (the thread-block tier of the reference's nested
-// parallelism, LONESTAR/rt/include/internal.h.prehip:99-158).
-constexpr uint32_t kCtaDegree = 256;
-constexpr uint32_t kCtaListCap = 256;
-
 template <int V>
 __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const SsspArgs& a, const Team team) {
   const DevCSR& g = a.g;
   const uint32_t tid = team.tid(), nthreads = team.nthreads();
+  __shared__ IdStage s_stage;
+  if (threadIdx.x == 0) stage_reset(s_stage);
   for (uint32_t v = tid; v < g.n; v += nthreads) {
     a.dist[v] = (v == a.src) ? 0 : kInf;
     a.mark[v] = 0;
@@ -764,7 +773,7 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
   }
   const uint32_t dsrc = g.row[a.src + 1] - g.row[a.src];
   if (tid == 0) {
-    const bool hub = dsrc > kBigDegree;
+    const bool hub = dsrc > kSsspBig;
     if (hub) a.hq[0][0] = a.src;
     else a.q[0][0] = a.src;
     for (int k = 0; k < 3; ++k) a.cnt[k].n_reg = a.cnt[k].n_big = a.cnt[k].m_next = 0;
@@ -774,6 +783,10 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
   }
   ok = bar.sync() && ok;
 
+  // graphs with fat rows probe a distance before every claim: most edges of a
+  // round improve nothing, and their hubs' atomics serialise on one address
+  // (R-MAT-17, a round of 15,640 vertices and 2.8 M edges)
+  const bool probe = g.m / kProbeMeanDegree >= g.n;
   // near threshold: vertices with dist < T are relaxed in the current bucket
   long long T = a.delta;
   uint32_t step = 1;       // index of the near counter set in use (rotating by 3)
@@ -823,8 +836,8 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
         }
         uint32_t d = 0;
         if (near) d = __ldg(g.row + v + 1) - __ldg(g.row + v);
-        warp_append(near && d <= kBigDegree, v, qout, &c->n_reg, g.n, a.overflow);
-        warp_append(near && d > kBigDegree, v, hout, &c->n_big, g.n, a.overflow);
+        warp_append(near && d <= kSsspBig, v, qout, &c->n_reg, g.n, a.overflow);
+        warp_append(near && d > kSsspBig, v, hout, &c->n_big, g.n, a.overflow);
         warp_append(keep, v, fout, fc_out, g.n, a.overflow);
       }
       fpar ^= 1;
@@ -856,34 +869,12 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
     uint32_t* fout = a.far[fpar];
     unsigned long long* fc = &a.fcnt[fpar];
     const uint32_t stamp = step + 1;  // stamps of vertices queued for the next round
-    unsigned long long my_edges = 0;
-    auto relax = [&](uint32_t u, uint32_t j, bool active) {
-      uint32_t v = 0;
-      bool to_near = false, to_far = false;
-      if (active) {
-        ++my_edges;
-        v = __ldg(g.dst + j);
-        const long long nd = (long long)__ldcg(a.dist + u) + (long long)__ldg(g.w + j);
-        if (nd < (long long)__ldcg(a.dist + v)) {
-          const int32_t old = atomicMin(a.dist + v, (int32_t)nd);
-          if (nd < (long long)old) {
-            if (nd < T) to_near = atomicExch(a.mark + v, stamp) != stamp;
-            else to_far = atomicExch(a.fmark + v, fgen) != fgen;
-          }
-        }
-      }
-      uint32_t d = 0;
-      if (to_near) d = __ldg(g.row + v + 1) - __ldg(g.row + v);
-      // (the near queue's slots may include reservation holes: 2n of them)
-      warp_append(to_near && d <= kBigDegree, v, qout, &c->n_reg, 2u * g.n, a.overflow);
-      warp_append(to_near && d > kBigDegree, v, hout, &c->n_big, g.n, a.overflow);
-      warp_append(to_far, v, fout, fc, g.n, a.overflow);
-    };
+    uint32_t my_edges = 0;
     // near-queue reservations in chunks of 64 slots when the queue (2n slots)
     // can hold the holes of every warp
     WarpRes res{0ull, 0u, 63ull * team.nwarps() <= g.n ? 64u : 0u};
-    const RelaxSink sink{qout, hout, &c->n_reg, &c->n_big, fout, fc, stamp, fgen, T, &res, 2u * g.n,
-                         nf > kPushPrecheckFrontier};
+    const RelaxSink sink{qout, hout, &c->n_reg, &c->n_big, fout, fc, stamp, fgen, (int32_t)min(T, (long long)kInf), &s_stage, &res, 2u * g.n,
+                         probe || nf > kPushPrecheckFrontier};
     // vertex lists relaxed edge-balanced: edge prefix, first edge, distance
     ListSmem& L_ = list_smem();
     uint32_t* s_lp = L_.p;
@@ -911,30 +902,24 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
       if (threadIdx.x == 0) s_lp[cnt] = carry;
       __syncthreads();
     };
-    if (nbig <= kHubList) {
-      // hubs: every CTA builds the same list; the team's threads share its edges
-      build_list([&](uint32_t i) { return __ldcg(hin + i); }, nbig);
-      sssp_relax_list(a, s_lp, s_lb, s_ld, nbig, team.tid(), team.nthreads(), sink, my_edges);
+    for (uint32_t h0 = 0; h0 < nbig; h0 += kHubList) {
+      // big vertices, kHubList at a time: every CTA builds the same list; the
+      // team's threads share its edges
+      const uint32_t cnt = min(nbig - h0, kHubList);
+      build_list([&](uint32_t i) { return __ldcg(hin + h0 + i); }, cnt);
+      sssp_relax_list(a, s_lp, s_lb, s_ld, cnt, team.tid(), team.nthreads(), sink, my_edges);
       __syncthreads();
-    } else {
-      expand_hubs(team, g, hin, nbig, relax);
     }
     {
-      // regular queue: vertices of degree > kCtaDegree go to the CTA's list
-      // (relaxed edge-balanced by the whole CTA below); degree > kWarpDegree
-      // edge-parallel across the warp; the rest one lane each; every tier
-      // keeps four edges per lane in flight
-      __shared__ uint32_t s_cta_u[kCtaListCap];
-      __shared__ uint32_t s_ncta;
-      if (threadIdx.x == 0) s_ncta = 0;
-      __syncthreads();
+      // regular queue, edge-balanced over each warp's group, four edges per
+      // lane in flight
       const uint32_t lane = lane_id();
-      const uint32_t gw = team.warp(), nwarps = team.nwarps();
-      for (uint32_t base = gw * 32u; base < nreg; base += nwarps * 32u) {
+      const uint32_t nwarps = team.nwarps(), gsz = group_size_of(nreg, nwarps);
+      for (uint32_t base = spread_warp(team) * gsz; base < nreg; base += nwarps * gsz) {
         const uint32_t i = base + lane;
         uint32_t u = 0, b = 0, e = 0;
         int32_t du0 = 0;
-        if (i < nreg) {
+        if (lane < gsz && i < nreg) {
           u = __ldcg(qin + i);
           if (u != kHole) {
             // the distance is read alongside the row range (one round trip):
@@ -944,36 +929,17 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
             du0 = __ldcg(a.dist + u);
           }
         }
-        const uint32_t deg = e - b;
-        bool warp_tier = deg > kWarpDegree;
-        if (deg > kCtaDegree) {
-          const uint32_t slot = atomicAdd(&s_ncta, 1u);
-          if (slot < kCtaListCap) {
-            s_cta_u[slot] = u;
-            warp_tier = false;
-          }
-        }
-        uint32_t coop = __ballot_sync(0xffffffffu, warp_tier);
-        while (coop) {
-          const int src = __ffs(coop) - 1;
-          coop &= coop - 1;
-          const uint32_t bb = __shfl_sync(0xffffffffu, b, src), ee = __shfl_sync(0xffffffffu, e, src);
-          const long long du = (long long)__shfl_sync(0xffffffffu, du0, src);
-          for (uint32_t j0 = bb; j0 < ee; j0 += 128) sssp_relax4(a, du, j0 + lane, 32u, ee, sink, my_edges);
-        }
-        const uint32_t mine = deg <= kWarpDegree ? deg : 0u;
-        const uint32_t kmax = warp_max_u32(mine);
-        const long long du = mine ? (long long)du0 : 0;
-        for (uint32_t k0 = 0; k0 < kmax; k0 += 4) sssp_relax4(a, du, b + k0, 1u, b + mine, sink, my_edges);
-      }
-      __syncthreads();
-      const uint32_t ncta = min(s_ncta, kCtaListCap);
-      if (ncta) {
-        build_list([&](uint32_t i) { return s_cta_u[i]; }, ncta);
-        sssp_relax_list(a, s_lp, s_lb, s_ld, ncta, threadIdx.x, blockDim.x, sink, my_edges);
+        auto step = [&](const uint32_t* j, const uint32_t* own, uint32_t act) {
+          int32_t du[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) du[r] = __shfl_sync(0xffffffffu, du0, own[r]);
+          sssp_relax4e(a, du, j, act, sink, my_edges);
+        };
+        walk_group(b, e - b, step);
       }
     }
     warp_res_close(qout, 2u * g.n, res, kHole);
+    stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow);
     relaxed_edges += my_edges;
     ++step;
     ok = bar.sync();
@@ -1015,16 +981,24 @@ struct BatchDesc {
   SsspArgs sssp;
 };
 
-template <int V>
+// One kernel per kind: a kernel holding both bodies spilled 1.4 KB a thread,
+// more than the L1 holds for a CTA (16 R-MAT SSSPs: 1.8 ms).  The descriptor is
+// copied to shared memory, so the body's reads of it cost no L2 trip.
+template <int V, int KIND>
 __global__ void __launch_bounds__(kGraphMaxThreads)
 batch_kernel(const BatchDesc* __restrict__ descs, const uint16_t* __restrict__ cta_inst) {
   __shared__ gsrb::BarrierShared bsh;
-  const uint32_t i = cta_inst[blockIdx.x];
-  const BatchDesc& d = descs[i];
+  __shared__ uint4 s_desc[(sizeof(BatchDesc) + 15) / 16];
+  static_assert(sizeof(BatchDesc) % 4 == 0, "copied word by word");
+  const uint32_t* src = reinterpret_cast<const uint32_t*>(descs + cta_inst[blockIdx.x]);
+  for (uint32_t i = threadIdx.x; i < sizeof(BatchDesc) / 4; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(s_desc)[i] = src[i];
+  __syncthreads();
+  const BatchDesc& d = *reinterpret_cast<const BatchDesc*>(s_desc);
   const Team team{blockIdx.x - d.first, d.count};
   gsrb::GridSync<V> bar;
   const bool ok = bar.init(d.gb, &bsh);
-  if (d.kind == 0) bfs_run<V>(bar, ok, d.bfs, team);
+  if (KIND == 0) bfs_run<V>(bar, ok, d.bfs, team);
   else sssp_run<V>(bar, ok, d.sssp, team);
   bar.finish();
 }
@@ -1277,6 +1251,14 @@ struct PrrArgs {
   uint32_t* out;        // [0] rounds, [1] worklist pushes (low 32 bits), [3] failure
   unsigned long long* out_edges;
 };
+
+// Vertices of the regular queue with more edges than this are pushed by their
+// whole CTA (after the CTA's warps have walked their queue groups), so that one
+// warp does not walk thousands of edges while the rest of the grid waits at
+// the round's barrier (the thread-block tier of the reference's nested
+// parallelism, LONESTAR/rt/include/internal.h.prehip:99-158).
+constexpr uint32_t kCtaDegree = 256;
+constexpr uint32_t kCtaListCap = 256;
 
 // Where a residual push step puts the vertices whose residual crossed epsilon.
 struct PrrSink {
@@ -1591,17 +1573,19 @@ const void* bfs_fn(int v) { return GSRB_GRAPH_FN(bfs_kernel)(v); }
 const void* sssp_fn(int v) { return GSRB_GRAPH_FN(sssp_kernel)(v); }
 const void* pr_fn(int v) { return GSRB_GRAPH_FN(pagerank_kernel)(v); }
 const void* prr_fn(int v) { return GSRB_GRAPH_FN(pr_residual_kernel)(v); }
-const void* batch_fn(int v) {
+template <int KIND>
+const void* batch_fn_k(int v) {
   switch (v) {  // variants without hardware cluster barriers (teams may be single CTAs)
-    case gsrb::V_SOFT2: return (const void*)batch_kernel<gsrb::V_SOFT2>;
-    case gsrb::V_FLAT: return (const void*)batch_kernel<gsrb::V_FLAT>;
-    case gsrb::V_TREE: return (const void*)batch_kernel<gsrb::V_TREE>;
-    case gsrb::V_FLIP: return (const void*)batch_kernel<gsrb::V_FLIP>;
-    case gsrb::V_FANOUT: return (const void*)batch_kernel<gsrb::V_FANOUT>;
-    case gsrb::V_HIER: return (const void*)batch_kernel<gsrb::V_HIER>;
+    case gsrb::V_SOFT2: return (const void*)batch_kernel<gsrb::V_SOFT2, KIND>;
+    case gsrb::V_FLAT: return (const void*)batch_kernel<gsrb::V_FLAT, KIND>;
+    case gsrb::V_TREE: return (const void*)batch_kernel<gsrb::V_TREE, KIND>;
+    case gsrb::V_FLIP: return (const void*)batch_kernel<gsrb::V_FLIP, KIND>;
+    case gsrb::V_FANOUT: return (const void*)batch_kernel<gsrb::V_FANOUT, KIND>;
+    case gsrb::V_HIER: return (const void*)batch_kernel<gsrb::V_HIER, KIND>;
     default: return nullptr;
   }
 }
+const void* batch_fn(int v, int kind) { return kind == 0 ? batch_fn_k<0>(v) : batch_fn_k<1>(v); }
 
 }  // namespace
 
@@ -2369,7 +2353,8 @@ struct gsrb_batch {
   gsrb_cfg_t cfg;
   int grid = 0;
   std::vector<uint32_t> first, count;
-  BatchDesc* h_desc = nullptr;  // pinned
+  BatchDesc* h_desc = nullptr;  // pinned; read by the last call's copy until `copied`
+  cudaEvent_t copied = nullptr;
   BatchDesc* d_desc = nullptr;
   uint16_t* d_cta_inst = nullptr;
 };
@@ -2444,11 +2429,12 @@ gsrb_status_t batch_launch(gsrb_batch* B, const uint32_t* srcs, int32_t* const* 
       if (st) return st;
     }
   gsrb_ctx* ctx = B->ctx;
-  const void* fn = batch_fn(B->cfg.variant);
+  const void* fn = batch_fn(B->cfg.variant, kind);
   if (!fn) return GSRB_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> g(ctx->mu);
+  std::vector<BatchDesc> desc((size_t)k);
   for (int i = 0; i < k; ++i) {
-    BatchDesc& d = B->h_desc[i];
+    BatchDesc& d = desc[i];
     memset(&d, 0, sizeof(d));
     // slot 1 + i and, for the group-counter variants, groups starting at the
     // instance's first CTA (an instance never has more groups than CTAs)
@@ -2466,7 +2452,19 @@ gsrb_status_t batch_launch(gsrb_batch* B, const uint32_t* srcs, int32_t* const* 
     }
     GSRB_CUDA(cudaMemsetAsync(B->graphs[i]->flags, 0, 128, ctx->stream));
   }
+  // The copy of an earlier call may not have run yet (calls are asynchronous):
+  // its source is rewritten only when the descriptors differ, and after it.
+  if (memcmp(B->h_desc, desc.data(), sizeof(BatchDesc) * (size_t)k) != 0) {
+    if (B->copied) GSRB_CUDA(cudaEventSynchronize(B->copied));
+    memcpy(B->h_desc, desc.data(), sizeof(BatchDesc) * (size_t)k);
+  }
   GSRB_CUDA(cudaMemcpyAsync(B->d_desc, B->h_desc, sizeof(BatchDesc) * k, cudaMemcpyHostToDevice, ctx->stream));
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  GSRB_CUDA(cudaStreamIsCapturing(ctx->stream, &capturing));
+  if (capturing == cudaStreamCaptureStatusNone) {
+    if (!B->copied) GSRB_CUDA(cudaEventCreateWithFlags(&B->copied, cudaEventDisableTiming));
+    GSRB_CUDA(cudaEventRecord(B->copied, ctx->stream));
+  }
   const BatchDesc* dd = B->d_desc;
   const uint16_t* ci = B->d_cta_inst;
   void* args[] = {(void*)&dd, (void*)&ci};
@@ -2487,7 +2485,7 @@ gsrb_status_t gsrb_batch_create(gsrb_ctx_t ctx, const gsrb_graph_t* graphs, int3
     c.threads = 512;
   }
   c.cluster = 1;
-  if (!batch_fn(c.variant)) return GSRB_ERR_UNSUPPORTED;
+  if (!batch_fn(c.variant, 0)) return GSRB_ERR_UNSUPPORTED;
   if (c.threads % 32 || c.threads > kGraphMaxThreads) return GSRB_ERR_ARG;
   const int grid = grid_of(ctx, c);
   if (grid < k || grid > 65535) return GSRB_ERR_ARG;
@@ -2533,6 +2531,7 @@ gsrb_status_t gsrb_batch_create(gsrb_ctx_t ctx, const gsrb_graph_t* graphs, int3
     f += cnt[i];
   }
   cudaError_t e = cudaMallocHost(&B->h_desc, sizeof(BatchDesc) * k);
+  if (!e) memset(B->h_desc, 0, sizeof(BatchDesc) * k);
   if (!e) e = cudaMalloc(&B->d_desc, sizeof(BatchDesc) * k);
   if (!e) e = cudaMalloc(&B->d_cta_inst, sizeof(uint16_t) * grid);
   if (!e) e = cudaMemcpy(B->d_cta_inst, inst.data(), sizeof(uint16_t) * grid, cudaMemcpyHostToDevice);
@@ -2547,6 +2546,7 @@ gsrb_status_t gsrb_batch_create(gsrb_ctx_t ctx, const gsrb_graph_t* graphs, int3
 gsrb_status_t gsrb_batch_free(gsrb_batch_t B) {
   if (!B) return GSRB_ERR_ARG;
   if (B->ctx) cudaStreamSynchronize(B->ctx->stream);
+  if (B->copied) cudaEventDestroy(B->copied);
   if (B->h_desc) cudaFreeHost(B->h_desc);
   if (B->d_desc) cudaFree(B->d_desc);
   if (B->d_cta_inst) cudaFree(B->d_cta_inst);

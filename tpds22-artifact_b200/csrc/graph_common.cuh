@@ -181,6 +181,84 @@ __device__ __forceinline__ void warp_res_close(T* q, uint32_t cap, WarpRes& res,
   res.left = 0;
 }
 
+// A CTA's queue entries of one round, collected in shared memory and written
+// to the queue at the round's end with one reservation on the shared counter
+// (stage_flush): an append costs a shared-memory atomic instead of a trip to
+// the L2, and the queue has no holes.  A round that outgrows the stage appends
+// the rest through the warps' reservations.
+template <class T, uint32_t CAP>
+struct Stage {
+  static constexpr uint32_t kCap = CAP;
+  T buf[CAP];
+  uint32_t n;      // entries asked for
+  uint32_t limit;  // first position of a warp that no longer fitted
+  uint32_t cnt;
+  unsigned long long base;
+};
+
+template <class T, uint32_t CAP>
+__device__ __forceinline__ void stage_reset(Stage<T, CAP>& st) {  // thread 0, before a CTA barrier
+  st.n = 0;
+  st.limit = CAP;
+}
+
+// Warp-synchronous; returns the number of entries that went past the stage.
+template <int K, class T, uint32_t CAP>
+__device__ __forceinline__ uint32_t stage_append(const bool* pred, const T* v, Stage<T, CAP>& st, T* q,
+                                                 unsigned long long* cnt, uint32_t cap, uint32_t res_cap,
+                                                 uint32_t* overflow, WarpRes& res, T hole) {
+  uint32_t mask[K];
+  uint32_t tot = 0;
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    mask[r] = __ballot_sync(0xffffffffu, pred[r]);
+    tot += __popc(mask[r]);
+  }
+  if (!tot) return 0;
+  uint32_t pos = 0;
+  if (lane_id() == 0) {
+    pos = atomicAdd(&st.n, tot);
+    if (pos + tot > CAP) atomicMin(&st.limit, pos);
+  }
+  pos = __shfl_sync(0xffffffffu, pos, 0);
+  if (pos + tot <= CAP) {
+    const uint32_t lt = lanemask_lt();
+#pragma unroll
+    for (int r = 0; r < K; ++r) {
+      if (pred[r]) st.buf[pos + __popc(mask[r] & lt)] = v[r];
+      pos += __popc(mask[r]);
+    }
+    return 0;
+  }
+  if (res.chunk) return warp_append_res<K>(pred, v, q, cnt, res_cap, overflow, res, hole);
+  warp_append_k<K>(pred, v, q, cnt, cap, overflow);
+  return tot;
+}
+
+// End of a round, by the whole CTA: the staged entries to the queue; leaves the
+// stage empty.
+template <class T, uint32_t CAP>
+__device__ __forceinline__ void stage_flush(Stage<T, CAP>& st, T* q, unsigned long long* cnt, uint32_t cap,
+                                            uint32_t* overflow) {
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const uint32_t k = min(st.n, st.limit);
+    st.base = k ? atomicAdd(cnt, (unsigned long long)k) : 0ull;
+    st.cnt = k;
+    stage_reset(st);
+  }
+  __syncthreads();
+  const uint32_t k = st.cnt;
+  for (uint32_t i = threadIdx.x; i < k; i += blockDim.x) {
+    const unsigned long long pos = st.base + i;
+    if (pos < cap) q[pos] = st.buf[i];
+    else atomicExch(overflow, 1u);
+  }
+}
+
+constexpr uint32_t kIdStage = 4096;
+using IdStage = Stage<uint32_t, kIdStage>;
+
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
@@ -427,6 +505,54 @@ __device__ __forceinline__ void bfs_push_lanes(const DevCSR& g, int32_t* level, 
     }
     push_append_reg<4>(reg, rg, s);
     if (__any_sync(0xffffffffu, any_big)) warp_append_k<4>(big, rg, s.hout, s.n_big, s.cap, s.overflow);
+  }
+}
+
+// Queue entries a warp takes at a time: 32, or fewer when the queue is too
+// short to give every warp of the team 32 (a round of 1000 vertices on 4736
+// warps: one each, so that no warp walks 32 vertices' edges while the others
+// wait at the round's barrier).
+__device__ __forceinline__ uint32_t group_size_of(uint32_t nq, uint32_t nwarps) {
+  const uint32_t per = (nq + nwarps - 1) / nwarps;
+  return per < 32u ? (per ? per : 1u) : 32u;
+}
+// The warp's place in the order in which groups are handed out: consecutive
+// groups go to different CTAs, so that a short queue reaches every SM.
+__device__ __forceinline__ uint32_t spread_warp(const Team& t) { return (threadIdx.x >> 5) * t.ncta + t.cta; }
+
+// Edge-balanced walk of a warp's group: lane l holds a range of `deg` edges
+// starting at b (0 edges: nothing).  The ranges are laid end to end and taken
+// 128 edges per step, four per lane, each lane finding its edge's owner by a
+// binary search over the lanes' exclusive prefix in registers:
+// step(j, own, act) gets the edge indices, the owning lanes and the mask of
+// valid ones.  A group costs ceil(edges / 128) steps whatever the degrees (one
+// lane or one warp per vertex costs up to a step per vertex).  Warp-synchronous.
+template <class F>
+__device__ __forceinline__ void walk_group(uint32_t b, uint32_t deg, F& step) {
+  const uint32_t lane = lane_id();
+  uint32_t inc = deg;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= (uint32_t)o) inc += y;
+  }
+  const uint32_t excl = inc - deg;
+  const uint32_t total = __shfl_sync(0xffffffffu, inc, 31);
+  const uint32_t first = b - excl;  // edge index of flat position f: first + f
+  for (uint32_t f0 = 0; f0 < total; f0 += 128) {
+    uint32_t j[4], own[4], act = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+      const uint32_t f = f0 + 32u * r + lane;
+      uint32_t o = 0;  // the last lane whose prefix is <= f (never a lane without edges)
+#pragma unroll
+      for (uint32_t st = 16; st > 0; st >>= 1)
+        if (__shfl_sync(0xffffffffu, excl, o + st) <= f) o += st;
+      own[r] = o;
+      j[r] = __shfl_sync(0xffffffffu, first, o) + f;
+      if (f < total) act |= 1u << r;
+    }
+    step(j, own, act);
   }
 }
 

@@ -78,3 +78,57 @@ def test_batch_calls_back_to_back(gsrb, ctx, orc, path_graphs):
     for i in range(6):
         for g, o in zip(gs, outs[i]):
             assert np.array_equal(o.download(), orc.dijkstra(g, i) if i % 2 else orc.bfs(g, i))
+
+
+def _thin_graphs(gsrb):
+    rng = np.random.default_rng(11)
+    n = 6000
+    # a chain of fans: levels of 1, then many, then 1 vertices (cluster -> grid -> cluster)
+    fans, src, dst, base = [40, 700, 30000, 3, 20000, 1], [], [], 0
+    for f in fans:
+        src.append(np.full(f, base))
+        dst.append(base + 1 + np.arange(f))
+        src.append(base + 1 + np.arange(f))
+        dst.append(np.full(f, base + f + 1))
+        base += f + 1
+    fan = gsrb.csr_from_edges(base + 1, np.concatenate(src), np.concatenate(dst))
+    # random tree plus chords: degrees 1 to about 12, long
+    par = np.maximum(0, np.arange(1, n) - 1 - rng.integers(0, 6, n - 1))
+    tree = gsrb.csr_from_edges(n, np.concatenate([par, rng.integers(0, n, 40)]),
+                               np.concatenate([np.arange(1, n), rng.integers(0, n, 40)]))
+    return {
+        "fans": fan,
+        "tree": tree,
+        "wide": gsrb.grid2d(3000, 40, seed=2),
+        "square": gsrb.grid2d(600, 600, seed=4),
+        "path": gsrb.csr_from_edges(5000, np.arange(4999), np.arange(1, 5000)),
+        "isolated": gsrb.csr_from_edges(70, [0, 1, 50], [1, 2, 51]),
+        "rmat": gsrb.rmat(15, 12, seed=8),
+        "directed": gsrb.csr_from_edges(4000, np.arange(3999), np.arange(1, 4000), symmetrize=False),
+    }
+
+
+@pytest.fixture(scope="module")
+def thin_graphs(gsrb):
+    return _thin_graphs(gsrb)
+
+
+@pytest.mark.parametrize("name", ["fans", "tree", "wide", "square", "path", "isolated", "rmat", "directed"])
+@pytest.mark.parametrize("variant", [None, 6, 8, 9])
+def test_bfs_thin_levels(gsrb, ctx, orc, thin_graphs, name, variant):
+    """Levels that run on one cluster, and the hand-overs between it and the grid."""
+    g = thin_graphs[name]
+    dg = ctx.graph(g)
+    out = ctx.array(g.nnodes, np.int32)
+    c = None if variant is None else gsrb.cfg(variant=variant, ctas_per_sm=1, threads=256)
+    for src in (0, g.nnodes // 2, g.nnodes - 1):
+        rc, st = dg.bfs(src, out, gsrb.BFS_HEURISTIC, c)
+        gsrb.check(rc, "bfs")
+        ctx.check_status("bfs")
+        want = orc.bfs(g, src)
+        assert np.array_equal(out.download(), want)
+        assert st.edges == orc.traversed_edges(g, want)
+        assert st.levels == int(want[want != 2**31 - 1].max()) + 1 if want.max() >= 0 else 0
+        tr = dg.trace()
+        assert tr["level"].tolist() == list(range(1, len(tr) + 1))
+        assert int(tr["nf"].sum()) == int((want != 2**31 - 1).sum())

@@ -14,6 +14,7 @@
 // reached in round L (bfs/kernel_gsrb.cu:299-311, :473-479, :724).
 #include "internal.h"
 #include "graph_common.cuh"
+#include "cluster_link.cuh"
 
 #include <algorithm>
 #include <string.h>
@@ -48,7 +49,20 @@ struct BfsArgs {
   uint32_t* lb_pre;    // [n] edge offset of each regular-queue entry
   uint32_t* lb_own;    // [m / kLbChunk + 2] entry owning each chunk's first edge
   uint32_t* lb_part;   // [kLbMaxCtas] per-CTA edge totals
+  uint32_t* phase;     // [0] PHASE_*, [1] policy decisions, [2] fallback level so far
+  bool staged;         // init kernel, then cluster and grid kernels in turn (a.phase says whose turn it is)
 };
+
+// Whose turn it is in a traversal that alternates between one cluster (thin
+// levels) and the whole grid (fat ones).
+enum : uint32_t { PHASE_GRID = 1, PHASE_DONE = 2, PHASE_CLUSTER = 3 };
+
+constexpr uint32_t kThinDegree = 8;           // graphs below this mean degree start and usually end on the cluster
+constexpr uint32_t kClQueue = 4096;           // entries per CTA and parity
+constexpr uint32_t kClMaxFrontier = 16384;    // larger levels go to the grid: past this 16 SMs' gathers
+constexpr uint32_t kClMaxEdges = 65536;       // (one a cycle and SM) cost more than a grid level
+constexpr uint32_t kClEnterFrontier = 2048;   // and come back below these
+constexpr unsigned long long kClEnterEdges = 8192;
 
 // Single-CTA phase: when a push level's frontier fits one pass of one CTA
 // (<= blockDim.x vertices and <= 4 blockDim.x out-edges) the heuristic and
@@ -101,7 +115,7 @@ __device__ __noinline__ void bfs_solo(const BfsArgs& a, uint32_t L, uint32_t nre
       m_acc += d;
     };
     expand_hub_ranges(one, hin, nbig, push_edge);
-    const PushSink sink{qout, hout, &s_c.n_reg, &s_c.n_big, g.n, a.overflow, nullptr, nullptr, 0u};
+    const PushSink sink{qout, hout, &s_c.n_reg, &s_c.n_big, g.n, a.overflow, nullptr, nullptr, 0u, nullptr};
     auto lanes = [&](uint32_t b, uint32_t mine, uint32_t kmax) {
       bfs_push_lanes(g, a.level, Li, b, mine, kmax, false, sink, m_acc);
     };
@@ -323,33 +337,49 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
   __shared__ uint32_t s_dir;
   __shared__ float s_pred;
   __shared__ MLPShared s_mlp;
+  __shared__ BfsStage s_stage;
   const DevCSR& g = a.g;
   const uint32_t tid = team.tid(), nthreads = team.nthreads();
+  if (threadIdx.x == 0) stage_reset(s_stage);
   if (a.mode == GSRB_BFS_LEARNED) mlp_stage(a.mlp, &s_mlp);  // visible after the barrier below
 
-  // init (bfs_init, bfs/kernel_gsrb.cu:299-311) fused into the persistent kernel
-  for (uint32_t v = tid; v < g.n; v += nthreads) a.level[v] = (v == a.src) ? 0 : kInf;
-  const uint32_t dsrc = g.row[a.src + 1] - g.row[a.src];
-  if (tid == 0) {
-    const bool hub = dsrc > kBigDegree;
-    reinterpret_cast<uint2*>(hub ? a.hq[0] : a.q[0])[0] = make_uint2(g.row[a.src], g.row[a.src + 1]);
-    a.cnt[0].n_reg = a.cnt[0].n_real = hub ? 0 : 1;
-    a.cnt[0].n_big = hub ? 1 : 0;
-    a.cnt[0].m_next = dsrc;
-    a.cnt[1].n_reg = a.cnt[1].n_real = a.cnt[1].n_big = a.cnt[1].m_next = 0;
-    a.cnt[2].n_reg = a.cnt[2].n_real = a.cnt[2].n_big = a.cnt[2].m_next = 0;
-  }
-  ok = bar.sync() && ok;
-
-  uint32_t nu = g.n - 1;
-  unsigned long long mu = (unsigned long long)g.m - dsrc;
-  unsigned long long edges = dsrc;
-  uint32_t dir = DIR_PUSH, prev_nf = 1;
-  bool fallback = a.mode != GSRB_BFS_LEARNED;
+  uint32_t nu, prev_nf = 1, L = 1, decisions = 0;
   uint32_t fb_level = 0;  // level at which the policy fell back (0 = never)
+  unsigned long long mu, edges;
+  if (a.staged) {
+    // the state is where the init kernel or the cluster left it
+    if (__ldcg(a.phase) != PHASE_GRID) return;
+    __syncthreads();  // the staged policy weights
+    L = __ldcg(a.solo + 0) + 1u;
+    nu = __ldcg(a.solo + 1);
+    prev_nf = __ldcg(a.solo + 2);
+    mu = __ldcg(reinterpret_cast<const unsigned long long*>(a.solo + 4));
+    edges = __ldcg(reinterpret_cast<const unsigned long long*>(a.solo + 6));
+    decisions = __ldcg(a.phase + 1);
+    fb_level = __ldcg(a.phase + 2);
+  } else {
+    // init (bfs_init, bfs/kernel_gsrb.cu:299-311) fused into the persistent kernel
+    for (uint32_t v = tid; v < g.n; v += nthreads) a.level[v] = (v == a.src) ? 0 : kInf;
+    const uint32_t dsrc = g.row[a.src + 1] - g.row[a.src];
+    if (tid == 0) {
+      const bool hub = dsrc > kBigDegree;
+      reinterpret_cast<uint2*>(hub ? a.hq[0] : a.q[0])[0] = make_uint2(g.row[a.src], g.row[a.src + 1]);
+      a.cnt[0].n_reg = a.cnt[0].n_real = hub ? 0 : 1;
+      a.cnt[0].n_big = hub ? 1 : 0;
+      a.cnt[0].m_next = dsrc;
+      a.cnt[1].n_reg = a.cnt[1].n_real = a.cnt[1].n_big = a.cnt[1].m_next = 0;
+      a.cnt[2].n_reg = a.cnt[2].n_real = a.cnt[2].n_big = a.cnt[2].m_next = 0;
+    }
+    ok = bar.sync() && ok;
+    nu = g.n - 1;
+    mu = (unsigned long long)g.m - dsrc;
+    edges = dsrc;
+  }
+  uint32_t dir = DIR_PUSH;
+  bool fallback = a.mode != GSRB_BFS_LEARNED || fb_level != 0;
   float pred = __int_as_float(0x7fc00000);
-  uint32_t L = 1;
-  uint32_t decisions = 0;
+  const uint32_t L0 = L;
+  bool to_cluster = false;
   uint32_t last_dir = DIR_PUSH, last_nf = 0;  // the policy's last decision and the frontier it saw
   unsigned long long last_mf = 0;
   for (; ok; ++L) {
@@ -360,11 +390,6 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
     const uint32_t nf = (uint32_t)cur.n_real + nbig;
     if (nf == 0) break;
     const unsigned long long mf = cur.m_next;
-    if (L > 1) {
-      nu -= nf;
-      mu -= mf;
-      edges += mf;
-    }
     // ---- choose the level's direction (identical in every CTA)
     if (!fallback && L > 1 && pred == pred) {
       const float actual = log2f(1.f + (float)nf);
@@ -372,6 +397,26 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
         fallback = true;
         fb_level = L;
       }
+    }
+    if (a.staged && L > L0 && nbig == 0 && nf <= kClEnterFrontier && mf <= kClEnterEdges) {
+      // a thin frontier goes to the cluster (after at least one level here)
+      if (tid == 0) {
+        a.solo[0] = L - 1;
+        a.solo[1] = nu;
+        a.solo[2] = prev_nf;
+        *reinterpret_cast<unsigned long long*>(a.solo + 4) = mu;
+        *reinterpret_cast<unsigned long long*>(a.solo + 6) = edges;
+        a.phase[0] = PHASE_CLUSTER;
+        a.phase[1] = decisions;
+        a.phase[2] = fb_level;
+      }
+      to_cluster = true;
+      break;
+    }
+    if (L > 1) {
+      nu -= nf;
+      mu -= mf;
+      edges += mf;
     }
     uint32_t nd = DIR_PUSH;
     if (a.mode == GSRB_BFS_PULL) {
@@ -439,7 +484,7 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
     }
     prev_nf = nf;
 
-    if (team.ncta > 1 && dir == DIR_PUSH && nf <= blockDim.x && mf <= 4ull * blockDim.x &&
+    if (!a.staged && team.ncta > 1 && dir == DIR_PUSH && nf <= blockDim.x && mf <= 4ull * blockDim.x &&
         (a.mode == GSRB_BFS_HEURISTIC || a.mode == GSRB_BFS_LEARNED)) {
       if (team.cta == 0) bfs_solo(a, L, nreg, nbig, nu, mu, edges, prev_nf);
       ok = bar.sync();
@@ -464,8 +509,10 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
     // regular-queue slots reserved per warp in chunks of 64 (one counter atomic
     // per chunk) when the queue's 2n slots can hold every warp's holes
     WarpRes res{0ull, 0u, 63ull * team.nwarps() <= g.n ? 64u : 0u};
-    uint32_t real_w = 0;  // regular entries this warp appended (warp-uniform)
-    const PushSink sink{qout, hout, &c->n_reg, &c->n_big, g.n, a.overflow, &res, &real_w, 2u * g.n};
+    const bool staged = mf >= kStageMinEdges;
+    uint32_t real_w = 0;  // regular entries this warp appended past the stage (warp-uniform)
+    const PushSink sink{qout, hout, &c->n_reg, &c->n_big, g.n, a.overflow, &res, &real_w, 2u * g.n,
+                        staged ? &s_stage : nullptr};
 
     auto discover = [&](bool disc, uint32_t v) {
       uint2 r = make_uint2(0u, 0u);
@@ -567,14 +614,19 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
         discover(found, v);
       }
     }
-    // per-warp edge sums and entry counts of the new frontier
+    // edge sums and entry counts of the new frontier; in a large level one
+    // update per CTA (one per warp made 4736 atomics on one line of the L2:
+    // R-MAT-22's first level 27.7 -> 16.3 us)
     warp_res_close(qout, 2u * g.n, res, make_uint2(0u, 0u));
     const unsigned long long ws = warp_sum_u64(m_acc);
-    if (lane_id() == 0 && ws) atomicAdd(&c->m_next, ws);
+    if (lane_id() == 0 && ws) atomicAdd(staged ? &s_stage.msum : &c->m_next, ws);
     if (lane_id() == 0 && real_w) atomicAdd(&c->n_real, (unsigned long long)real_w);
+    if (staged) stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, &c->n_real, &c->m_next);
     ok = bar.sync();
   }
+  if (to_cluster) return;
   if (team.cta == 0 && threadIdx.x == 0) {
+    if (a.staged) a.phase[0] = PHASE_DONE;
     a.out[0] = L - 1;  // levels with a non-empty frontier beyond the source
     a.out[2] = decisions;
     a.out[3] = ok ? 0u : 1u;
@@ -584,6 +636,308 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
   // register: scanning the trace for it here cost one thread a dependent load
   // per level (about 1 ms on a 4095-level mesh)
   if (team.cta == 0 && threadIdx.x == 0 && a.mode == GSRB_BFS_LEARNED) a.out[1] = fb_level;
+}
+
+// ---- thin levels on one cluster ---------------------------------------------
+// A 2048^2 grid has 4073 levels of at most 2051 vertices: on the grid a level
+// cost 11.4 us at 2 x 512 threads per SM, of which the barrier is two and the
+// rest the chain of trips to L2.  Here a level is: entry (shared memory) ->
+// destinations -> claims with the candidates' row ranges -> shared-memory
+// append -> records exchanged, about 1200 cycles.
+struct BfsClShared {
+  uint2 q[2][kClQueue];  // edge ranges of the frontier's vertices, by parity of the level
+  ClusterLink link;
+  uint32_t n[2];      // entries asked for in the level being built, by parity
+  uint32_t extra[2];  // entries that went to the global queues
+  uint32_t empty[2];  // slots they left empty here
+  uint32_t m[2];      // their out-edges
+  uint32_t fat[2];    // bit 0: an entry of more than 4 edges, bit 1: of more than 8
+};
+
+// Bulk prefetches of an array into L2, 4 KiB each (whole 16-byte units inside it).
+__device__ __forceinline__ void prefetch_l2(const void* array, uint64_t bytes, uint32_t tid, uint32_t nt) {
+  const uint64_t a0 = (uint64_t)array, b = (a0 + 15) & ~15ull, e = (a0 + bytes) & ~15ull;
+  for (uint64_t at = b + (uint64_t)tid * 4096; at < e; at += (uint64_t)nt * 4096) {
+    const uint32_t len = (uint32_t)min((uint64_t)4096, e - at);
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(at), "r"(len) : "memory");
+  }
+}
+
+// Level, queue and counter set-up of a traversal that starts on the cluster
+// or (hub sources) on the grid; the CSR of a thin graph is brought into L2, so
+// that a level's misses do not wait for DRAM in turn (prefetch != 0).
+__global__ void __launch_bounds__(512) bfs_init_kernel(BfsArgs a, uint32_t* flags, uint32_t prefetch) {
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  const DevCSR& g = a.g;
+  for (uint32_t v = tid; v < g.n; v += nt) a.level[v] = v == a.src ? 0 : kInf;
+  if (tid == 0) {
+    for (int k = 0; k < 32; ++k) flags[k] = 0;
+    const uint32_t b = g.row[a.src], e = g.row[a.src + 1];
+    const bool hub = e - b > kBigDegree;
+    reinterpret_cast<uint2*>(hub ? a.hq[0] : a.q[0])[0] = make_uint2(b, e);
+    for (int k = 0; k < 3; ++k) a.cnt[k].n_reg = a.cnt[k].n_real = a.cnt[k].n_big = a.cnt[k].m_next = 0;
+    a.cnt[0].n_reg = a.cnt[0].n_real = hub ? 0 : 1;
+    a.cnt[0].n_big = hub ? 1 : 0;
+    a.cnt[0].m_next = e - b;
+    a.solo[1] = g.n - 1;
+    a.solo[2] = 1;
+    *reinterpret_cast<unsigned long long*>(a.solo + 4) = (unsigned long long)g.m - (e - b);
+    *reinterpret_cast<unsigned long long*>(a.solo + 6) = e - b;
+    // (the policy decides a traversal's first level: that one runs on the grid)
+    a.phase[0] = e - b > kClEnterEdges || hub || a.mode == GSRB_BFS_LEARNED ? PHASE_GRID : PHASE_CLUSTER;
+  }
+  if (prefetch) {
+    prefetch_l2(g.row, (uint64_t)(g.n + 1) * 4, tid, nt);
+    prefetch_l2(g.dst, (uint64_t)g.m * 4, tid, nt);
+  }
+}
+
+// K edges per lane (bit r of `act`: edge j[r]): destinations, claims
+// (compare-and-swap INF -> L, with the row ranges of the candidates), append.
+// Warp-synchronous.
+template <int K>
+__device__ __forceinline__ void bfs_cl_push(const BfsArgs& a, BfsClShared& s, uint32_t L, const uint32_t* j,
+                                            uint32_t act) {
+  const DevCSR& g = a.g;
+  const uint32_t p = L & 1u;
+  uint32_t v[K];
+  int32_t old[K];
+  uint2 rg[K];
+#pragma unroll
+  for (int r = 0; r < K; ++r) v[r] = ((act >> r) & 1u) ? __ldg(g.dst + j[r]) : 0u;
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    old[r] = 0;
+    if ((act >> r) & 1u) old[r] = atomicCAS(a.level + v[r], kInf, (int32_t)L);
+  }
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    rg[r] = make_uint2(0u, 0u);
+    if ((act >> r) & 1u) rg[r] = make_uint2(__ldg(g.row + v[r]), __ldg(g.row + v[r] + 1));
+  }
+  uint32_t mask[K], tot = 0, m_acc = 0, dmax = 0;
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    const bool disc = ((act >> r) & 1u) && old[r] == kInf;
+    if (!disc) rg[r] = make_uint2(0u, 0u);
+    const uint32_t d = rg[r].y - rg[r].x;
+    // the first edges are on their way to the SM while the level ends
+    if (d) asm volatile("prefetch.global.L1 [%0];" ::"l"(g.dst + rg[r].x));
+    dmax = max(dmax, d);
+    m_acc += d;
+    mask[r] = __ballot_sync(0xffffffffu, disc);
+    tot += __popc(mask[r]);
+  }
+  if (!tot) return;
+  const uint32_t lane = lane_id();
+  uint32_t pos = 0;
+  if (lane == 0) pos = atomicAdd(&s.n[p], tot);
+  m_acc = __reduce_add_sync(0xffffffffu, m_acc);
+  const bool fat = __any_sync(0xffffffffu, dmax > 4u);
+  if (lane == 0) atomicAdd(&s.m[p], m_acc);
+  pos = __shfl_sync(0xffffffffu, pos, 0);
+  bool hub = false;
+  if (fat) {
+    hub = __any_sync(0xffffffffu, dmax > kBigDegree);
+    const bool fat8 = __any_sync(0xffffffffu, dmax > 8u);
+    if (lane == 0) atomicOr(&s.fat[p], fat8 ? 3u : 1u);
+  }
+  const uint32_t lt = lanemask_lt();
+  if (pos + tot <= kClQueue && !hub) {
+#pragma unroll
+    for (int r = 0; r < K; ++r) {
+      if ((mask[r] >> lane) & 1u) s.q[p][pos + __popc(mask[r] & lt)] = rg[r];
+      pos += __popc(mask[r]);
+    }
+    return;
+  }
+  // no room left, or a hub: these go to the global queues and the level that
+  // follows to the grid.  The slots reserved above stay empty ranges.
+  const uint32_t left = pos < kClQueue ? min(tot, kClQueue - pos) : 0u;
+  for (uint32_t k = lane; k < left; k += 32) s.q[p][pos + k] = make_uint2(0u, 0u);
+  LevelCounters* c = &a.cnt[L % 3];
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    const bool disc = (mask[r] >> lane) & 1u, big = rg[r].y - rg[r].x > kBigDegree;
+    warp_append(disc && !big, rg[r], reinterpret_cast<uint2*>(a.q[p]), &c->n_reg, 2u * a.g.n, a.overflow);
+    warp_append(disc && big, rg[r], reinterpret_cast<uint2*>(a.hq[p]), &c->n_big, a.g.n, a.overflow);
+  }
+  if (lane == 0) {
+    atomicAdd(&s.extra[p], tot);
+    atomicAdd(&s.empty[p], left);
+  }
+}
+
+// A level over the CTA's own entries, all of at most 1 << SH edges: K edges per
+// lane, (1 << SH) / K lanes per entry.  A level is a chain of dependent
+// instructions as much as of trips to L2, so one edge per lane (fewer
+// instructions per warp on more warps) wins while one pass takes them all, and
+// two per lane over two passes of one.
+template <int SH, int K>
+__device__ __forceinline__ void bfs_cl_thin(const BfsArgs& a, BfsClShared& s, uint32_t L, uint32_t own) {
+  constexpr int kSh = K == 1 ? SH : SH - 1;  // log2 of the lanes per entry
+  const uint32_t p = (L - 1) & 1u;
+  for (uint32_t i = threadIdx.x; ((i - lane_id()) >> kSh) < own; i += blockDim.x) {
+    uint2 r = make_uint2(0u, 0u);
+    if ((i >> kSh) < own) r = s.q[p][i >> kSh];
+    uint32_t j[K], act = 0;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      j[k] = r.x + (i & ((1u << kSh) - 1u)) * K + k;
+      if (j[k] < r.y) act |= 1u << k;
+    }
+    bfs_cl_push<K>(a, s, L, j, act);
+  }
+}
+
+__global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, unsigned long long timeout_ns) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  BfsClShared& s = *reinterpret_cast<BfsClShared*>(cl_smem);
+  if (__ldcg(a.phase) != PHASE_CLUSTER) return;  // the same in every CTA
+  const uint32_t rank = gsrb::ptx::cluster_ctarank(), ncta = gsrb::ptx::cluster_nctarank();
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  uint32_t L = __ldcg(a.solo + 0) + 1u, nu = __ldcg(a.solo + 1), prev_nf = __ldcg(a.solo + 2);
+  unsigned long long mu = __ldcg(reinterpret_cast<const unsigned long long*>(a.solo + 4));
+  unsigned long long edges = __ldcg(reinterpret_cast<const unsigned long long*>(a.solo + 6));
+  uint32_t nf = (uint32_t)__ldcg(&a.cnt[(L - 1) % 3].n_real);
+  unsigned long long mf = __ldcg(&a.cnt[(L - 1) % 3].m_next);
+  const uint32_t slots = (uint32_t)__ldcg(&a.cnt[(L - 1) % 3].n_reg);
+  if (threadIdx.x == 0) {
+    link_init(s.link);
+    s.n[0] = s.n[1] = s.extra[0] = s.extra[1] = s.empty[0] = s.empty[1] = s.m[0] = s.m[1] = 0;
+    s.fat[0] = s.fat[1] = 3u;  // of the entries read below nothing is known
+  }
+  gsrb::ptx::cluster_sync();  // also: every CTA has read the counters
+  if (rank == 0 && threadIdx.x < 3)
+    a.cnt[threadIdx.x].n_reg = a.cnt[threadIdx.x].n_real = a.cnt[threadIdx.x].n_big = a.cnt[threadIdx.x].m_next = 0;
+  // this CTA's part of the frontier (holes and isolated vertices dropped; at
+  // most kClEnterFrontier entries in all)
+  uint32_t p = (L - 1) & 1u;
+  {
+    const uint2* qg = reinterpret_cast<const uint2*>(a.q[p]);
+    const uint32_t s0 = (uint32_t)((uint64_t)slots * rank / ncta), s1 = (uint32_t)((uint64_t)slots * (rank + 1) / ncta);
+    for (uint32_t i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
+      const uint2 r = __ldcg(qg + i);
+      if (r.y != r.x) s.q[p][atomicAdd(&s.n[p], 1u)] = r;
+    }
+  }
+  uint32_t phases = 0, fl = 0, own;
+  bool ok, first = true;
+  // the last warp of CTA 0 (idle in thin levels) keeps the traversal's account
+  const bool books = rank == 0 && wid == nw - 1;
+  if (threadIdx.x == 0) link_expect(s.link, p, ncta);
+  __syncthreads();
+  if (wid == 0) link_publish(s.link, p, make_uint4(s.n[p], 0u, 0u, 0u), rank, ncta);
+  for (;;) {
+    // the frontier of level L - 1 is in q[p], its records in tab[p]
+    ok = link_wait(s.link, p, phases, timeout_ns);
+    const LinkSum t = link_sum(s.link, p, rank, ncta);
+    own = t.own;
+    if (!first) {
+      nf = t.x + t.y;
+      mf = t.z;
+      fl = t.any ? 1u : 0u;
+    }
+    if (!ok || nf == 0 || fl || nf > kClMaxFrontier || (uint32_t)mf > kClMaxEdges) break;
+    first = false;
+    const uint32_t o = L & 1u;  // the level being built
+    const uint32_t fat = s.fat[p];  // (cleared for level L + 1 in level L's tail)
+    if (threadIdx.x == 0) {
+      // published; next used in level L + 1, after this level's barrier
+      s.n[p] = s.extra[p] = s.empty[p] = s.m[p] = 0;
+      link_expect(s.link, o, ncta);
+    }
+    if (books) {
+      if (L > 1) {
+        nu -= nf;
+        mu -= mf;
+        edges += mf;
+      }
+      prev_nf = nf;
+      if (lane == 0 && L - 1 < a.trace_cap) {
+        LevelTrace r;
+        r.level = L;
+        r.dir = 3u;  // push outside the grid's level loop
+        r.nf = nf;
+        r.nu = nu;
+        r.mf = mf;
+        r.mu = mu;
+        r.t_ns = gsrb::ptx::globaltimer_ns();
+        r.pred = __int_as_float(0x7fc00000);
+        r.fallback = 0u;
+        a.trace[L - 1] = r;
+      }
+    }
+    auto step = [&](const uint32_t* j, const uint32_t*, uint32_t act) { bfs_cl_push<4>(a, s, L, j, act); };
+    if (link_uneven(t, ncta)) {
+      // redistribute: an equal slice of all entries, read from their CTAs
+      gsrb::ptx::cluster_sync();
+      const uint32_t i0 = (uint32_t)((uint64_t)t.x * rank / ncta), i1 = (uint32_t)((uint64_t)t.x * (rank + 1) / ncta);
+      const uint32_t gsz = cl_group(i1 - i0);
+      for (uint32_t base = i0 + wid * gsz; base < i1; base += nw * gsz) {
+        const bool in = lane < gsz && base + lane < i1;
+        const uint32_t at = link_locate(s.link, p, ncta, in ? base + lane : 0u);
+        uint2 r = make_uint2(0u, 0u);
+        if (in)
+          r = ld_cluster_v2(gsrb::ptx::mapa_shared(gsrb::ptx::smem_u32(&s.q[p][at & 0xffffu]), at >> 16));
+        walk_group(r.x, r.y - r.x, step);
+      }
+    } else if (fat == 0u) {
+      if (own <= kClThreads / 4) bfs_cl_thin<2, 1>(a, s, L, own);
+      else bfs_cl_thin<2, 2>(a, s, L, own);
+    } else if (fat == 1u) {
+      bfs_cl_thin<3, 2>(a, s, L, own);
+    } else {
+      const uint32_t gsz = cl_group(own);
+      for (uint32_t base = wid * gsz; base < own; base += nw * gsz) {
+        uint2 r = make_uint2(0u, 0u);
+        if (lane < gsz && base + lane < own) r = s.q[p][base + lane];
+        walk_group(r.x, r.y - r.x, step);
+      }
+    }
+    __syncthreads();
+    if (wid == 0) {
+      // slots (past the queue's end the entries went to the global queue), the
+      // entries beyond them (less the empty slots), edges, any in the global queue
+      if (lane == 0) s.fat[p] = 0;  // every thread has read it; next set in level L + 1
+      const uint32_t k = min(s.n[o], kClQueue);
+      link_publish(s.link, o, make_uint4(k, s.extra[o] - s.empty[o], s.m[o], s.extra[o]), rank, ncta);
+    }
+    p = o;
+    ++L;
+  }
+  if (nf == 0 || !ok) {
+    if (books && lane == 0) {
+      a.out[0] = L - 1;
+      a.out[1] = __ldcg(a.phase + 2);
+      a.out[2] = __ldcg(a.phase + 1);
+      a.out[3] = ok ? 0u : 1u;
+      *a.out_edges = edges;
+      a.phase[0] = PHASE_DONE;
+    }
+  } else {
+    // hand the frontier of level L - 1 to the grid
+    LevelCounters* c = &a.cnt[(L - 1) % 3];
+    __shared__ unsigned long long s_base;
+    if (threadIdx.x == 0) s_base = atomicAdd(&c->n_reg, (unsigned long long)own);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < own; i += blockDim.x) {
+      const unsigned long long at = s_base + i;
+      if (at < 2ull * a.g.n) reinterpret_cast<uint2*>(a.q[p])[at] = s.q[p][i];
+      else atomicExch(a.overflow, 1u);
+    }
+    if (books && lane == 0) {
+      c->n_real = nf - (uint32_t)__ldcg(&c->n_big);
+      c->m_next = mf;
+      a.solo[0] = L - 1;
+      a.solo[1] = nu;
+      a.solo[2] = prev_nf;
+      *reinterpret_cast<unsigned long long*>(a.solo + 4) = mu;
+      *reinterpret_cast<unsigned long long*>(a.solo + 6) = edges;
+      a.phase[0] = PHASE_GRID;
+    }
+  }
+  gsrb::ptx::cluster_sync();  // no CTA leaves while a record to it may be in flight
 }
 
 constexpr int kGraphMaxThreads = 1024;
@@ -939,7 +1293,7 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
       }
     }
     warp_res_close(qout, 2u * g.n, res, kHole);
-    stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow);
+    stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
     relaxed_edges += my_edges;
     ++step;
     ok = bar.sync();
@@ -1866,12 +2220,22 @@ gsrb_cfg_t graph_cfg(gsrb_ctx* ctx, const gsrb_cfg_t* in) {
   return c;
 }
 
+// CTAs of the cluster that runs thin steps: 16, 8 where 16 cannot be placed,
+// 0 where neither can.
+int cluster_ctas(gsrb_ctx* ctx, const void* fn, size_t smem) {
+  for (int k = (int)kClMaxCtas; k >= 8; k /= 2) {
+    int cap = 0;
+    if (coresident_ctas(ctx, fn, (int)kClThreads, smem, k, &cap) == GSRB_OK && cap >= k) return k;
+  }
+  return 0;
+}
+
 gsrb_status_t finish_stats(gsrb_graph* G, gsrb_traversal_stats_t* st, float ms) {
   uint32_t h[32];
   unsigned long long edges = 0;
   GSRB_CUDA(cudaStreamSynchronize(G->ctx->stream));
   GSRB_CUDA(cudaMemcpy(h, G->flags, sizeof(h), cudaMemcpyDeviceToHost));
-  GSRB_CUDA(cudaMemcpy(&edges, (char*)G->flags + 64, sizeof(edges), cudaMemcpyDeviceToHost));
+  memcpy(&edges, h + 16, sizeof(edges));
   if (st) {
     st->levels = h[4];
     st->aux = h[5];
@@ -2180,17 +2544,61 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
   a.out = G->flags + 4;
   a.out_edges = (unsigned long long*)((char*)G->flags + 64);
   a.solo = G->flags + 8;
+  a.phase = G->flags + 20;
   G->last_delta = 0;
   std::lock_guard<std::mutex> g(ctx->mu);
-  GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
   gsrb::GridBarrier gb = make_barrier(ctx, c, 0, (uint32_t)grid, 0, 0);
   void* args[] = {&gb, &a};
   if (!ctx->events[62]) GSRB_CUDA(cudaEventCreate(&ctx->events[62]));
   if (!ctx->events[63]) GSRB_CUDA(cudaEventCreate(&ctx->events[63]));
+  // The schedules that choose per level run thin levels on one cluster.
+  const int ncl = mode == GSRB_BFS_HEURISTIC || mode == GSRB_BFS_LEARNED
+                      ? cluster_ctas(ctx, (const void*)bfs_cluster_kernel, sizeof(BfsClShared))
+                      : 0;
+  a.staged = ncl > 0;
   GSRB_CUDA(cudaEventRecord(ctx->events[62], ctx->stream));
-  gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
-  if (st) return st;
-  GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
+  gsrb_status_t st = GSRB_OK;
+  if (!a.staged) {
+    GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
+    st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
+    if (st) return st;
+    GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
+  } else {
+    uint32_t* flags = G->flags;
+    // mean degree < kThinDegree and a CSR that leaves L2 room for the levels:
+    // bring it in
+    const bool thin = G->m / kThinDegree < G->n;
+    uint32_t prefetch = thin && ((uint64_t)G->m + G->n) * 4 <= (uint64_t)ctx->l2_bytes / 4 * 3 ? 1u : 0u;
+    void* iargs[] = {&a, &flags, &prefetch};
+    st = launch_plain(ctx, (const void*)bfs_init_kernel, dim3(ctx->num_sms * 2), dim3(512), 0, iargs);
+    if (st) return st;
+    unsigned long long timeout_ns = gb.timeout_ns;
+    void* cargs[] = {&a, &timeout_ns};
+    auto cluster = [&] {
+      return launch_persistent(ctx, (const void*)bfs_cluster_kernel, ncl, kClThreads, sizeof(BfsClShared), ncl, 0,
+                               cargs);
+    };
+    auto whole = [&] { return launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args); };
+    // A kernel whose turn it is not returns at once, so the usual order is
+    // queued without a look at the device: the cluster for the whole of a thin
+    // graph; cluster, grid and the thin last levels on the cluster again
+    // otherwise (no cluster first for a source of more edges than it takes, or
+    // when the policy decides the first level).
+    const bool cluster_first = mode != GSRB_BFS_LEARNED && G->h_row[src + 1] - G->h_row[src] <= kClEnterEdges;
+    if (cluster_first) st = cluster();
+    for (uint32_t turn = thin && cluster_first ? 0u : 1u;; ++turn) {
+      if (!st && turn) st = whole();
+      if (!st && turn) st = cluster();
+      if (st) return st;
+      GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
+      uint32_t phase = 0;
+      GSRB_CUDA(cudaMemcpyAsync(&phase, a.phase, sizeof(phase), cudaMemcpyDeviceToHost, ctx->stream));
+      GSRB_CUDA(cudaStreamSynchronize(ctx->stream));
+      if (phase == PHASE_DONE) break;
+      // (every turn runs at least one level; n levels are the most there are)
+      if ((phase != PHASE_GRID && phase != PHASE_CLUSTER) || turn > G->n) return GSRB_ERR_STATE;
+    }
+  }
   GSRB_CUDA(cudaEventSynchronize(ctx->events[63]));
   float ms = 0;
   GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
@@ -2386,6 +2794,8 @@ BfsArgs bfs_args(gsrb_graph* G, uint32_t src, int32_t* level, int32_t mode) {
   a.lb_pre = G->lb_pre;
   a.lb_own = G->lb_own;
   a.lb_part = G->lb_part;
+  a.phase = G->flags + 20;
+  a.staged = false;
   return a;
 }
 

@@ -192,17 +192,19 @@ struct Stage {
   T buf[CAP];
   uint32_t n;      // entries asked for
   uint32_t limit;  // first position of a warp that no longer fitted
-  uint32_t cnt;
+  uint32_t cnt, pad;
   unsigned long long base;
+  unsigned long long msum;  // BFS: out-edges of the entries appended by the CTA
 };
 
 template <class T, uint32_t CAP>
 __device__ __forceinline__ void stage_reset(Stage<T, CAP>& st) {  // thread 0, before a CTA barrier
   st.n = 0;
   st.limit = CAP;
+  st.msum = 0;
 }
 
-// Warp-synchronous; returns the number of entries that went past the stage.
+// Returns the number of entries that went past the stage.  Warp-synchronous.
 template <int K, class T, uint32_t CAP>
 __device__ __forceinline__ uint32_t stage_append(const bool* pred, const T* v, Stage<T, CAP>& st, T* q,
                                                  unsigned long long* cnt, uint32_t cap, uint32_t res_cap,
@@ -236,13 +238,16 @@ __device__ __forceinline__ uint32_t stage_append(const bool* pred, const T* v, S
 }
 
 // End of a round, by the whole CTA: the staged entries to the queue; leaves the
-// stage empty.
+// stage empty.  `real` (may be null) counts the entries, `msum` (may be null)
+// receives the CTA's out-edge sum.
 template <class T, uint32_t CAP>
 __device__ __forceinline__ void stage_flush(Stage<T, CAP>& st, T* q, unsigned long long* cnt, uint32_t cap,
-                                            uint32_t* overflow) {
+                                            uint32_t* overflow, unsigned long long* real, unsigned long long* msum) {
   __syncthreads();
   if (threadIdx.x == 0) {
     const uint32_t k = min(st.n, st.limit);
+    if (msum && st.msum) atomicAdd(msum, st.msum);
+    if (real && k) atomicAdd(real, (unsigned long long)k);
     st.base = k ? atomicAdd(cnt, (unsigned long long)k) : 0ull;
     st.cnt = k;
     stage_reset(st);
@@ -256,7 +261,8 @@ __device__ __forceinline__ void stage_flush(Stage<T, CAP>& st, T* q, unsigned lo
   }
 }
 
-constexpr uint32_t kIdStage = 4096;
+constexpr uint32_t kBfsStage = 2048, kIdStage = 4096;
+using BfsStage = Stage<uint2, kBfsStage>;
 using IdStage = Stage<uint32_t, kIdStage>;
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
@@ -376,15 +382,20 @@ struct PushSink {
   uint32_t cap;
   uint32_t* overflow;
   WarpRes* res;                // regular-queue reservation (null: append directly)
-  uint32_t* real;              // regular entries appended by this warp (with res)
+  uint32_t* real;              // regular entries this warp appended past the stage (with res)
   uint32_t rcap;               // regular-queue slots (with res)
+  BfsStage* stage;             // the CTA's stage (null: small level)
 };
 
-// Appends the regular entries of a push step: through the warp's reservation
-// when there is one (counting the entries), else directly.
+// Appends the regular entries of a push step: to the CTA's stage, through the
+// warp's reservation (small levels; both count the entries that went past the
+// stage), or directly in the single-CTA phase.
 template <int K>
 __device__ __forceinline__ void push_append_reg(const bool* reg, const uint2* rg, const PushSink& s) {
-  if (s.res && s.res->chunk) {
+  if (s.stage) {
+    *s.real += stage_append<K>(reg, rg, *s.stage, s.qout, s.n_reg, s.cap, s.rcap, s.overflow, *s.res,
+                               make_uint2(0u, 0u));
+  } else if (s.res && s.res->chunk) {
     *s.real += warp_append_res<K>(reg, rg, s.qout, s.n_reg, s.rcap, s.overflow, *s.res, make_uint2(0u, 0u));
   } else {
     if (s.real) {
@@ -396,6 +407,11 @@ __device__ __forceinline__ void push_append_reg(const bool* reg, const uint2* rg
     warp_append_k<K>(reg, rg, s.qout, s.n_reg, s.cap, s.overflow);
   }
 }
+
+// Levels with at least this many frontier edges collect their entries in the
+// CTAs' stages; in smaller ones a warp appends about once, and the flush at the
+// level's end would only add a trip (2048^2 grid: 44.1 ms staged, 41.1 not).
+constexpr unsigned long long kStageMinEdges = 16384;
 
 // Frontiers up to this size check a destination's level only through the
 // claim itself (compare-and-swap INF -> L) and load its row range alongside

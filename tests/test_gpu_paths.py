@@ -132,3 +132,20 @@ def test_bfs_thin_levels(gsrb, ctx, orc, thin_graphs, name, variant):
         tr = dg.trace()
         assert tr["level"].tolist() == list(range(1, len(tr) + 1))
         assert int(tr["nf"].sum()) == int((want != 2**31 - 1).sum())
+
+
+@pytest.mark.parametrize("name", ["fans", "tree", "wide", "square", "path", "isolated", "directed"])
+@pytest.mark.parametrize("delta", [40, 1000, 1 << 30])
+def test_sssp_thin_graphs(gsrb, ctx, orc, thin_graphs, name, delta):
+    """Thin graphs: rounds on one cluster, and the hand-over of the rest to the
+    grid (the fans outgrow the cluster's queues, the wide buckets its far piles)."""
+    g = thin_graphs[name]
+    dg = ctx.graph(g)
+    out = ctx.array(g.nnodes, np.int32)
+    for src in (0, g.nnodes // 2):
+        rc, st = dg.sssp(src, out, delta)
+        gsrb.check(rc, "sssp")
+        ctx.check_status("sssp")
+        want = orc.dijkstra(g, src)
+        assert np.array_equal(out.download(), want)
+        assert st.levels >= 1 and st.edges >= orc.traversed_edges(g, want) and st.delta == delta

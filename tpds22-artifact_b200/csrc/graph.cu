@@ -771,11 +771,12 @@ __device__ __forceinline__ void bfs_cl_push(const BfsArgs& a, BfsClShared& s, ui
 // A level over the CTA's own entries, all of at most 1 << SH edges: K edges per
 // lane, (1 << SH) / K lanes per entry.  A level is a chain of dependent
 // instructions as much as of trips to L2, so one edge per lane (fewer
-// instructions per warp on more warps) wins while one pass takes them all, and
-// two per lane over two passes of one.
+// instructions per warp on more warps) wins while one pass takes them all, then
+// two per lane over two passes of one (2048^2 grid 9.6 -> 8.7 ms; four measured
+// the same as two).
 template <int SH, int K>
 __device__ __forceinline__ void bfs_cl_thin(const BfsArgs& a, BfsClShared& s, uint32_t L, uint32_t own) {
-  constexpr int kSh = K == 1 ? SH : SH - 1;  // log2 of the lanes per entry
+  constexpr int kSh = SH - (K - 1);  // log2 of the lanes per entry
   const uint32_t p = (L - 1) & 1u;
   for (uint32_t i = threadIdx.x; ((i - lane_id()) >> kSh) < own; i += blockDim.x) {
     uint2 r = make_uint2(0u, 0u);
@@ -970,6 +971,9 @@ struct SsspArgs {
   int32_t delta;
   uint32_t* out;        // [0] relax rounds, [1] buckets, [3] failure
   unsigned long long* out_edges;
+  uint32_t* phase;      // [0] PHASE_*
+  uint32_t* state;      // where the cluster left off: [0] rounds, [1] buckets, [2..3] near threshold
+  bool staged;          // init and cluster kernels before the grid kernel (a.phase says whether it has work)
 };
 
 // Vertices of more edges than this go to the near hub queue and are relaxed
@@ -977,6 +981,7 @@ struct SsspArgs {
 // per CTA above 256, R-MAT-17's second round waited for the CTAs whose share of
 // the frontier held the most edges: 93 -> 66 us).
 constexpr uint32_t kSsspBig = 256;
+constexpr uint32_t kSsspStep = 2;         // the grid's first step after the cluster (queue parity, counter set, stamp)
 constexpr uint32_t kProbeMeanDegree = 8;  // graphs of this mean degree probe before claiming in every round
 
 // Where an SSSP relax step puts the vertices whose distance it lowered.
@@ -1120,33 +1125,42 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
   const uint32_t tid = team.tid(), nthreads = team.nthreads();
   __shared__ IdStage s_stage;
   if (threadIdx.x == 0) stage_reset(s_stage);
-  for (uint32_t v = tid; v < g.n; v += nthreads) {
-    a.dist[v] = (v == a.src) ? 0 : kInf;
-    a.mark[v] = 0;
-    a.fmark[v] = 0;
+  uint32_t step = 1;       // index of the near counter set in use (rotating by 3)
+  uint32_t rounds = 0, buckets = 1;
+  // near threshold: vertices with dist < T are relaxed in the current bucket
+  long long T = a.delta;
+  if (a.staged) {
+    if (__ldcg(a.phase) != PHASE_GRID) return;
+    __syncthreads();  // the stage is empty
+    step = kSsspStep;
+    rounds = __ldcg(a.state + 0);
+    buckets = __ldcg(a.state + 1);
+    T = __ldcg(reinterpret_cast<const long long*>(a.state + 2));
+  } else {
+    for (uint32_t v = tid; v < g.n; v += nthreads) {
+      a.dist[v] = (v == a.src) ? 0 : kInf;
+      a.mark[v] = 0;
+      a.fmark[v] = 0;
+    }
+    const uint32_t dsrc = g.row[a.src + 1] - g.row[a.src];
+    if (tid == 0) {
+      const bool hub = dsrc > kSsspBig;
+      if (hub) a.hq[0][0] = a.src;
+      else a.q[0][0] = a.src;
+      for (int k = 0; k < 3; ++k) a.cnt[k].n_reg = a.cnt[k].n_big = a.cnt[k].m_next = 0;
+      a.cnt[0].n_reg = hub ? 0 : 1;
+      a.cnt[0].n_big = hub ? 1 : 0;
+      a.fcnt[0] = a.fcnt[1] = 0;
+    }
+    ok = bar.sync() && ok;
   }
-  const uint32_t dsrc = g.row[a.src + 1] - g.row[a.src];
-  if (tid == 0) {
-    const bool hub = dsrc > kSsspBig;
-    if (hub) a.hq[0][0] = a.src;
-    else a.q[0][0] = a.src;
-    for (int k = 0; k < 3; ++k) a.cnt[k].n_reg = a.cnt[k].n_big = a.cnt[k].m_next = 0;
-    a.cnt[0].n_reg = hub ? 0 : 1;
-    a.cnt[0].n_big = hub ? 1 : 0;
-    a.fcnt[0] = a.fcnt[1] = 0;
-  }
-  ok = bar.sync() && ok;
 
   // graphs with fat rows probe a distance before every claim: most edges of a
   // round improve nothing, and their hubs' atomics serialise on one address
   // (R-MAT-17, a round of 15,640 vertices and 2.8 M edges)
   const bool probe = g.m / kProbeMeanDegree >= g.n;
-  // near threshold: vertices with dist < T are relaxed in the current bucket
-  long long T = a.delta;
-  uint32_t step = 1;       // index of the near counter set in use (rotating by 3)
   uint32_t fpar = 0;       // far pile parity
   uint32_t fgen = 1;       // generation of the current far pile (fmark stamps: a vertex enters a pile once)
-  uint32_t rounds = 0, buckets = 1;
   unsigned long long relaxed_edges = 0;
   while (ok) {
     const LevelCounters cur = {__ldcg(&a.cnt[(step - 1) % 3].n_reg), __ldcg(&a.cnt[(step - 1) % 3].n_big), 0, 0};
@@ -1306,6 +1320,343 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
     a.out[1] = buckets;
     a.out[3] = ok ? 0u : 1u;
   }
+}
+
+// ---- thin graphs on one cluster ------------------------------------------------
+// The rounds of a mesh's SSSP relax a few thousand edges: as in
+// bfs_cluster_kernel the near queue stays in shared memory and the step's
+// records are its barrier, and so do the far piles.  An entry carries the
+// distance it was queued with: one that no longer equals the vertex's distance
+// is skipped (whoever lowered it queued another entry), so no stamps are
+// exchanged.  When a round outgrows the cluster the rest of the traversal runs
+// on the grid (2048^2 grid, 5000 rounds: at most 10,000 entries).
+constexpr uint32_t kSsspClQueue = 3072;   // near entries per CTA and parity
+constexpr uint32_t kSsspClFar = 4096;     // far entries per CTA and parity
+constexpr uint32_t kSsspClDegree = 1024;  // vertices of more edges go to the grid's team-wide lists
+
+struct SsspClShared {
+  uint4 q[2][kSsspClQueue];  // {vertex, first edge, end, distance} by parity of the step
+  uint2 far[2][kSsspClFar];  // {vertex, distance}
+  ClusterLink link;
+  uint32_t n[2];     // near slots asked for, by parity of the step being built
+  uint32_t m[2];     // their edges
+  uint32_t fat[2];   // bit 0: an entry of more than 4 edges, bit 1: of more than 8
+  uint32_t leave[2]; // an entry went to the global queues
+  uint32_t farn[2];  // far slots asked for, by far parity
+};
+
+__global__ void __launch_bounds__(512) sssp_init_kernel(SsspArgs a, uint32_t* flags, uint32_t prefetch) {
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+  const DevCSR& g = a.g;
+  for (uint32_t v = tid; v < g.n; v += nt) {
+    a.dist[v] = v == a.src ? 0 : kInf;
+    a.mark[v] = 0;
+    a.fmark[v] = 0;
+  }
+  if (tid == 0) {
+    for (int k = 0; k < 32; ++k) flags[k] = 0;
+    for (int k = 0; k < 3; ++k) a.cnt[k].n_reg = a.cnt[k].n_big = a.cnt[k].m_next = 0;
+    a.fcnt[0] = a.fcnt[1] = 0;
+    const uint32_t d = g.row[a.src + 1] - g.row[a.src];
+    if (d > kSsspClDegree) {  // the grid's queues of its first step
+      a.hq[(kSsspStep - 1) & 1][0] = a.src;
+      a.cnt[(kSsspStep - 1) % 3].n_big = 1;
+    }
+    a.state[1] = 1;
+    *reinterpret_cast<long long*>(a.state + 2) = a.delta;
+    a.phase[0] = d > kSsspClDegree ? PHASE_GRID : PHASE_CLUSTER;
+  }
+  if (prefetch) {
+    prefetch_l2(g.row, (uint64_t)(g.n + 1) * 4, tid, nt);
+    prefetch_l2(g.dst, (uint64_t)g.m * 4, tid, nt);
+    prefetch_l2(g.w, (uint64_t)g.m * 4, tid, nt);
+  }
+}
+
+// To the grid's queues of step kSsspStep, each vertex once.  Warp-synchronous.
+__device__ __forceinline__ void sssp_to_grid_near(const SsspArgs& a, bool pred, uint32_t v, uint32_t deg) {
+  constexpr uint32_t p = (kSsspStep - 1) & 1u;
+  LevelCounters* c = &a.cnt[(kSsspStep - 1) % 3];
+  if (pred) pred = atomicExch(a.mark + v, kSsspStep) != kSsspStep;
+  warp_append(pred && deg <= kSsspBig, v, a.q[p], &c->n_reg, 2u * a.g.n, a.overflow);
+  warp_append(pred && deg > kSsspBig, v, a.hq[p], &c->n_big, a.g.n, a.overflow);
+}
+__device__ __forceinline__ void sssp_to_grid_far(const SsspArgs& a, bool pred, uint32_t v) {
+  if (pred) pred = atomicExch(a.fmark + v, 1u) != 1u;  // the grid's first far generation
+  warp_append(pred, v, a.far[0], &a.fcnt[0], a.g.n, a.overflow);
+}
+
+// Appends lane entries to the near queue being built (parity o) / the far pile f.
+__device__ __forceinline__ void sssp_cl_near(const SsspArgs& a, SsspClShared& s, uint32_t o, bool pred, uint4 e) {
+  const uint32_t mask = __ballot_sync(0xffffffffu, pred);
+  if (!mask) return;
+  const uint32_t lane = lane_id(), tot = __popc(mask), d = pred ? e.z - e.y : 0u;
+  uint32_t pos = 0;
+  if (lane == 0) pos = atomicAdd(&s.n[o], tot);
+  const uint32_t m = __reduce_add_sync(0xffffffffu, d);
+  if (lane == 0) atomicAdd(&s.m[o], m);
+  const bool fat = __any_sync(0xffffffffu, d > 4u);
+  pos = __shfl_sync(0xffffffffu, pos, 0);
+  bool hub = false;
+  if (fat) {
+    hub = __any_sync(0xffffffffu, d > kSsspClDegree);
+    const bool fat8 = __any_sync(0xffffffffu, d > 8u);
+    if (lane == 0) atomicOr(&s.fat[o], fat8 ? 3u : 1u);
+  }
+  const uint32_t at = pos + __popc(mask & lanemask_lt());
+  if (pos + tot <= kSsspClQueue && !hub) {
+    if (pred) s.q[o][at] = e;
+    return;
+  }
+  // no room, or a vertex for the grid: the slots reserved here stay empty
+  if (pred && at < kSsspClQueue) s.q[o][at] = make_uint4(0u, 0u, 0u, 0u);
+  sssp_to_grid_near(a, pred, e.x, d);
+  if (lane == 0) atomicOr(&s.leave[o], 1u);
+}
+__device__ __forceinline__ void sssp_cl_far(const SsspArgs& a, SsspClShared& s, uint32_t o, uint32_t f, bool pred,
+                                            uint32_t v, int32_t d) {
+  const uint32_t mask = __ballot_sync(0xffffffffu, pred);
+  if (!mask) return;
+  const uint32_t tot = __popc(mask);
+  uint32_t pos = 0;
+  if (lane_id() == 0) pos = atomicAdd(&s.farn[f], tot);
+  pos = __shfl_sync(0xffffffffu, pos, 0);
+  const uint32_t at = pos + __popc(mask & lanemask_lt());
+  if (pred && at < kSsspClFar) s.far[f][at] = make_uint2(v, (uint32_t)d);
+  if (pos + tot <= kSsspClFar) return;
+  sssp_to_grid_far(a, pred && at >= kSsspClFar, v);
+  if (lane_id() == 0) atomicOr(&s.leave[o], 1u);
+}
+
+// K edges per lane (bit r of `act`: edge j[r]) of entries at distance du[r],
+// current when cur[r] still equals it.  Warp-synchronous.
+template <int K>
+__device__ __forceinline__ void sssp_cl_push(const SsspArgs& a, SsspClShared& s, uint32_t o, uint32_t f, int32_t T,
+                                             const uint32_t* j, const int32_t* du, const int32_t* cur, uint32_t act,
+                                             uint32_t& relaxed) {
+  const DevCSR& g = a.g;
+  uint32_t v[K];
+  int32_t nd[K], old[K];
+  uint2 rg[K];
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    v[r] = 0;
+    nd[r] = 0;
+    if ((act >> r) & 1u) {
+      v[r] = __ldg(g.dst + j[r]);
+      nd[r] = __ldg(g.w + j[r]);
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    nd[r] = add_sat(du[r], nd[r]);
+    const bool on = ((act >> r) & 1u) && cur[r] == du[r];
+    relaxed += on;
+    if (!on || nd[r] == kInf) act &= ~(1u << r);
+    old[r] = 0;
+    if ((act >> r) & 1u) old[r] = atomicMin(a.dist + v[r], nd[r]);
+  }
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    rg[r] = make_uint2(0u, 0u);
+    if (((act >> r) & 1u) && nd[r] < T) rg[r] = make_uint2(__ldg(g.row + v[r]), __ldg(g.row + v[r] + 1));
+  }
+#pragma unroll
+  for (int r = 0; r < K; ++r) {
+    const bool imp = ((act >> r) & 1u) && nd[r] < old[r], near = imp && nd[r] < T;
+    if (near) {  // the first edges are on their way to the SM while the round ends
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(g.dst + rg[r].x));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(g.w + rg[r].x));
+    }
+    sssp_cl_near(a, s, o, near, make_uint4(v[r], rg[r].x, rg[r].y, (uint32_t)nd[r]));
+    sssp_cl_far(a, s, o, f, imp && !near, v[r], nd[r]);
+  }
+}
+
+// A round over the CTA's own entries, all of at most 1 << SH edges (see bfs_cl_thin).
+template <int SH, int K>
+__device__ __forceinline__ void sssp_cl_thin(const SsspArgs& a, SsspClShared& s, uint32_t p, uint32_t f, int32_t T,
+                                             uint32_t own, uint32_t& relaxed) {
+  constexpr int kSh = SH - (K - 1);
+  for (uint32_t i = threadIdx.x; ((i - lane_id()) >> kSh) < own; i += blockDim.x) {
+    uint4 e = make_uint4(0u, 0u, 0u, 0u);
+    if ((i >> kSh) < own) e = s.q[p][i >> kSh];
+    uint32_t j[K], act = 0;
+    int32_t du[K], cur[K];
+    int32_t c = -1;
+    if (e.y < e.z) c = __ldcg(a.dist + e.x);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      j[k] = e.y + (i & ((1u << kSh) - 1u)) * K + k;
+      if (j[k] < e.z) act |= 1u << k;
+      du[k] = (int32_t)e.w;
+      cur[k] = c;
+    }
+    sssp_cl_push<K>(a, s, p ^ 1u, f, T, j, du, cur, act, relaxed);
+  }
+}
+
+__global__ void __launch_bounds__(kClThreads, 1) sssp_cluster_kernel(SsspArgs a, unsigned long long timeout_ns) {
+  extern __shared__ __align__(16) unsigned char cl_smem[];
+  SsspClShared& s = *reinterpret_cast<SsspClShared*>(cl_smem);
+  if (__ldcg(a.phase) != PHASE_CLUSTER) return;  // the same in every CTA
+  const DevCSR& g = a.g;
+  const uint32_t rank = gsrb::ptx::cluster_ctarank(), ncta = gsrb::ptx::cluster_nctarank();
+  const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (threadIdx.x == 0) {
+    link_init(s.link);
+    s.n[0] = s.n[1] = s.m[0] = s.m[1] = s.leave[0] = s.leave[1] = s.farn[0] = s.farn[1] = 0;
+    s.fat[0] = s.fat[1] = 3u;  // nothing is known of the source
+    if (rank == 0) {
+      s.q[0][0] = make_uint4(a.src, g.row[a.src], g.row[a.src + 1], 0u);
+      s.n[0] = 1;
+    }
+    link_expect(s.link, 0u, ncta);
+  }
+  gsrb::ptx::cluster_sync();
+  if (wid == 0) link_publish(s.link, 0u, make_uint4(s.n[0], 0u, 0u, 0u), rank, ncta);
+  uint32_t phases = 0, p = 0, f = 0, rounds = 0, buckets = 1, own, relaxed = 0;
+  unsigned long long edges = 0;
+  long long T = a.delta;
+  const bool books = rank == 0 && wid == nw - 1;
+  bool ok, done = false;
+  for (;;) {
+    // this step's near entries are in q[p], the far pile in far[f]
+    ok = link_wait(s.link, p, phases, timeout_ns);
+    const LinkSum t = link_sum(s.link, p, rank, ncta);
+    own = t.own;
+    const bool leave = __any_sync(0xffffffffu, lane < ncta && s.link.tab[p][lane].w != 0u);
+    if (!ok || leave || t.x > kClMaxFrontier || t.z > kClMaxEdges) break;
+    if (t.x == 0 && t.y == 0) {
+      done = true;
+      break;
+    }
+    const uint32_t o = p ^ 1u;
+    const uint32_t fat = s.fat[p];
+    if (threadIdx.x == 0) {
+      s.n[p] = s.m[p] = s.leave[p] = 0;  // published; next used in the step after this one
+      link_expect(s.link, o, ncta);
+    }
+    if (t.x == 0) {
+      // near bucket empty: advance the threshold and refill from the far piles
+      T += a.delta;
+      ++buckets;
+      const int32_t T32 = (int32_t)min(T, (long long)kInf);
+      const uint32_t nfar = min(s.farn[f], kSsspClFar);
+      for (uint32_t base = wid * 32u; base < nfar; base += nw * 32u) {
+        uint2 e = make_uint2(0u, 0u);
+        bool live = base + lane < nfar;
+        if (live) {
+          e = s.far[f][base + lane];
+          live = __ldcg(a.dist + e.x) == (int32_t)e.y;  // else lowered since: queued elsewhere
+        }
+        const bool near = live && (int32_t)e.y < T32;
+        uint2 rg = make_uint2(0u, 0u);
+        if (near) rg = make_uint2(__ldg(g.row + e.x), __ldg(g.row + e.x + 1));
+        sssp_cl_near(a, s, o, near, make_uint4(e.x, rg.x, rg.y, e.y));
+        sssp_cl_far(a, s, o, f ^ 1u, live && !near, e.x, (int32_t)e.y);
+      }
+      f ^= 1u;
+    } else {
+      ++rounds;
+      if (books && lane == 0 && rounds - 1 < a.trace_cap) {
+        LevelTrace r;
+        r.level = rounds;
+        r.dir = 3u;
+        r.nf = t.x;
+        r.nu = buckets;
+        r.mf = 0;
+        r.mu = (unsigned long long)T;
+        r.t_ns = gsrb::ptx::globaltimer_ns();
+        r.pred = __int_as_float(0x7fc00000);
+        r.fallback = 0;
+        a.trace[rounds - 1] = r;
+      }
+      const int32_t T32 = (int32_t)min(T, (long long)kInf);
+      auto group = [&](uint4 e) {
+        int32_t c = -1;
+        if (e.y < e.z) c = __ldcg(a.dist + e.x);
+        auto step = [&](const uint32_t* j, const uint32_t* from, uint32_t act) {
+          int32_t du[4], cur[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            du[r] = __shfl_sync(0xffffffffu, (int32_t)e.w, from[r]);
+            cur[r] = __shfl_sync(0xffffffffu, c, from[r]);
+          }
+          sssp_cl_push<4>(a, s, o, f, T32, j, du, cur, act, relaxed);
+        };
+        walk_group(e.y, e.z - e.y, step);
+      };
+      if (link_uneven(t, ncta)) {
+        // redistribute: an equal slice of all entries, read from their CTAs
+        gsrb::ptx::cluster_sync();
+        const uint32_t i0 = (uint32_t)((uint64_t)t.x * rank / ncta);
+        const uint32_t i1 = (uint32_t)((uint64_t)t.x * (rank + 1) / ncta);
+        const uint32_t gsz = cl_group(i1 - i0);
+        for (uint32_t base = i0 + wid * gsz; base < i1; base += nw * gsz) {
+          const bool in = lane < gsz && base + lane < i1;
+          const uint32_t at = link_locate(s.link, p, ncta, in ? base + lane : 0u);
+          uint4 e = make_uint4(0u, 0u, 0u, 0u);
+          if (in)
+            e = ld_cluster_v4(gsrb::ptx::mapa_shared(gsrb::ptx::smem_u32(&s.q[p][at & 0xffffu]), at >> 16));
+          group(e);
+        }
+      } else if (fat == 0u) {
+        if (own <= kClThreads / 4) sssp_cl_thin<2, 1>(a, s, p, f, T32, own, relaxed);
+        else sssp_cl_thin<2, 2>(a, s, p, f, T32, own, relaxed);
+      } else {
+        const uint32_t gsz = cl_group(own);
+        for (uint32_t base = wid * gsz; base < own; base += nw * gsz) {
+          uint4 e = make_uint4(0u, 0u, 0u, 0u);
+          if (lane < gsz && base + lane < own) e = s.q[p][base + lane];
+          group(e);
+        }
+      }
+      if (relaxed >= 1u << 30) {
+        edges += relaxed;
+        relaxed = 0;
+      }
+    }
+    __syncthreads();
+    if (wid == 0) {
+      if (lane == 0) {
+        s.fat[p] = 0;  // every thread has read it
+        if (t.x == 0) s.farn[f ^ 1u] = 0;  // the pile just read
+      }
+      link_publish(s.link, o, make_uint4(min(s.n[o], kSsspClQueue), min(s.farn[f], kSsspClFar), s.m[o], s.leave[o]),
+                   rank, ncta);
+    }
+    p = o;
+  }
+  edges = warp_sum_u64(edges + relaxed);
+  if (lane == 0 && edges) atomicAdd(a.out_edges, edges);
+  if (!done && ok) {
+    // the grid takes over: this step's entries and the far piles, each vertex once
+    for (uint32_t base = wid * 32u; base < own; base += nw * 32u) {
+      uint4 e = make_uint4(0u, 0u, 0u, 0u);
+      if (base + lane < own) e = s.q[p][base + lane];
+      sssp_to_grid_near(a, e.y < e.z, e.x, e.z - e.y);
+    }
+    const uint32_t nfar = min(s.farn[f], kSsspClFar);
+    for (uint32_t base = wid * 32u; base < nfar; base += nw * 32u) {
+      uint2 e = make_uint2(0u, 0u);
+      if (base + lane < nfar) e = s.far[f][base + lane];
+      sssp_to_grid_far(a, base + lane < nfar, e.x);
+    }
+  }
+  if (books && lane == 0) {
+    if (done || !ok) {
+      a.out[0] = rounds;
+      a.out[1] = buckets;
+      a.out[3] = ok ? 0u : 1u;
+    } else {
+      a.state[0] = rounds;
+      a.state[1] = buckets;
+      *reinterpret_cast<long long*>(a.state + 2) = T;
+    }
+    a.phase[0] = done || !ok ? PHASE_DONE : PHASE_GRID;
+  }
+  gsrb::ptx::cluster_sync();  // no CTA leaves while a record to it may be in flight
 }
 
 template <int V>
@@ -2646,15 +2997,36 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
   a.delta = delta;
   a.out = G->flags + 4;
   a.out_edges = (unsigned long long*)((char*)G->flags + 64);
+  a.phase = G->flags + 20;
+  a.state = G->flags + 8;
   G->last_delta = delta;
   std::lock_guard<std::mutex> g(ctx->mu);
-  GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
+  // thin graphs (mean degree < kThinDegree) start on one cluster; the grid
+  // kernel queued behind it returns at once unless the traversal outgrew it
+  const int ncl = G->m / kThinDegree < G->n
+                      ? cluster_ctas(ctx, (const void*)sssp_cluster_kernel, sizeof(SsspClShared))
+                      : 0;
+  a.staged = ncl > 0;
   gsrb::GridBarrier gb = make_barrier(ctx, c, 0, (uint32_t)grid, 0, 0);
   void* args[] = {&gb, &a};
   if (!ctx->events[62]) GSRB_CUDA(cudaEventCreate(&ctx->events[62]));
   if (!ctx->events[63]) GSRB_CUDA(cudaEventCreate(&ctx->events[63]));
   GSRB_CUDA(cudaEventRecord(ctx->events[62], ctx->stream));
-  gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
+  gsrb_status_t st = GSRB_OK;
+  if (!a.staged) {
+    GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
+  } else {
+    uint32_t* flags = G->flags;
+    uint32_t prefetch = ((uint64_t)G->m * 2 + G->n) * 4 <= (uint64_t)ctx->l2_bytes / 4 * 3 ? 1u : 0u;
+    void* iargs[] = {&a, &flags, &prefetch};
+    st = launch_plain(ctx, (const void*)sssp_init_kernel, dim3(ctx->num_sms * 2), dim3(512), 0, iargs);
+    if (st) return st;
+    unsigned long long timeout_ns = gb.timeout_ns;
+    void* cargs[] = {&a, &timeout_ns};
+    st = launch_persistent(ctx, (const void*)sssp_cluster_kernel, ncl, kClThreads, sizeof(SsspClShared), ncl, 0, cargs);
+    if (st) return st;
+  }
+  st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
   GSRB_CUDA(cudaEventSynchronize(ctx->events[63]));
@@ -2819,6 +3191,9 @@ SsspArgs sssp_args(gsrb_graph* G, uint32_t src, int32_t* dist, int32_t delta) {
   a.delta = delta;
   a.out = G->flags + 4;
   a.out_edges = (unsigned long long*)((char*)G->flags + 64);
+  a.phase = G->flags + 20;
+  a.state = G->flags + 8;
+  a.staged = false;
   return a;
 }
 

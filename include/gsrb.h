@@ -184,13 +184,16 @@ gsrb_status_t gsrb_reduce_i32(gsrb_ctx_t ctx, const int32_t* d_in, size_t n, int
  * occupancy check before it cannot see other processes' kernels). */
 gsrb_status_t gsrb_reduce_i32_noalloc(const int32_t* d_in, size_t n, int64_t* d_out, void* stream);
 
-/* ---- scan (three-phase persistent exclusive prefix sum) ---------------------------
- * Exclusive prefix sum, one persistent launch (default one 1024-thread CTA per
- * SM).  The input is walked in segments of one chunk per CTA (cfg->tile
- * elements, 0 = 32768); per segment: chunk sums, one split-phase grid barrier
- * that overlaps the next segment's reads, then the chunk is re-read from L2,
- * scanned and written.  uint32 wraps around like the reference's
- * cpu_sum_scan; the FP32 variant keeps chunk offsets in FP64.
+/* ---- scan (persistent exclusive prefix sum) ------------------------------------
+ * Exclusive prefix sum, one persistent launch.  cfg == NULL and 16-byte aligned
+ * arrays: the streaming form (one CTA per SM; every element read and written
+ * once; tile sums exchanged in tagged words instead of at a grid barrier).
+ * Otherwise (default one 1024-thread CTA per SM) the input is walked in
+ * segments of one chunk per CTA (cfg->tile elements, 0 = 32768); per segment:
+ * chunk sums, one split-phase grid barrier that overlaps the next segment's
+ * reads, then the chunk is re-read from L2, scanned and written.  uint32 wraps
+ * around like the reference's cpu_sum_scan; the FP32 variant keeps chunk and
+ * tile offsets in FP64.  The order of additions is fixed in both forms.
  * In-place (d_in == d_out) is allowed.  Replaces gpu_prescan /
  * sum_scan_blelloch of scan/scan_gsrb.cu:486-804 (API scan/scan.h:16-18).
  * Asynchronous. */

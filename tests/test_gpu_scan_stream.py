@@ -1,0 +1,81 @@
+"""The default scan (streaming form) against the CPU oracle: tile edges,
+remainders, alignment, in place, chains of calls and graph replay."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# tiles are 2048 elements up to 148 of them, 8192 above; copies are whole 16-byte units
+SIZES = [1, 3, 4, 5, 2047, 2048, 2049, 6 * 2048 + 1, 148 * 2048 - 1, 148 * 2048, 148 * 2048 + 1,
+         148 * 8192 * 6 + 8191, 148 * 8192 * 9 + 2]
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_scan_u32_default(gsrb, ctx, orc, n):
+    rng = np.random.default_rng(n)
+    a = rng.integers(0, 2**32, n, dtype=np.uint32)  # wraps around
+    d, o = ctx.to_device(a), ctx.array(n, np.uint32)
+    want = orc.scan_u32(a)
+    for _ in range(2):
+        gsrb.check(ctx.scan(d, o, n), "scan")
+    ctx.check_status("scan")
+    assert np.array_equal(o.download(), want)
+    gsrb.check(ctx.scan(d, d, n), "scan in place")
+    ctx.check_status("scan")
+    assert np.array_equal(d.download(), want)
+
+
+@pytest.mark.parametrize("n", SIZES)
+def test_scan_f32_default(gsrb, ctx, orc, n):
+    a = gsrb.uniform_f32(n, n)
+    d, o = ctx.to_device(a), ctx.array(n, np.float32)
+    gsrb.check(ctx.scan(d, o, n), "scan")
+    ctx.check_status("scan")
+    first = o.download()
+    ref = orc.scan_f32_f64(a)
+    # FP32 within a warp's 128 elements (seven roundings), FP64 between, one rounding of the result
+    assert np.all(np.abs(first - ref) <= 8 * 2.0**-24 * np.maximum(ref, 2.0**-24) + 1e-30)
+    gsrb.check(ctx.scan(d, o, n), "scan")
+    assert np.array_equal(o.download(), first)  # the same bits every time
+
+
+@pytest.mark.parametrize("ioff,ooff", [(1, 0), (0, 1), (2, 2), (4, 0), (0, 4)])
+def test_scan_alignment(gsrb, ctx, orc, ioff, ooff):
+    n = 30011
+    a = np.arange(n + 8, dtype=np.uint32)
+    d, o = ctx.to_device(a), ctx.array(n + 8, np.uint32)
+    o.upload(np.full(n + 8, 7, np.uint32))
+    gsrb.check(ctx.scan(d.at(ioff), o.at(ooff), n), "scan")
+    ctx.check_status("scan")
+    got = o.download()
+    assert np.array_equal(got[ooff:ooff + n], orc.scan_u32(a[ioff:ioff + n]))
+    assert np.all(got[:ooff] == 7) and np.all(got[ooff + n:] == 7)
+
+
+def test_scan_chain_and_replay(gsrb, ctx, orc):
+    """Each call reads what the one before wrote, of several sizes, plain and replayed."""
+    sizes = [100_003, 2048 * 148 + 5, 3_000_001, 17, 800_000]
+    n = max(sizes)
+    a = np.random.default_rng(1).integers(0, 2**32, n, dtype=np.uint32)
+    want = a.copy()
+    for k in sizes:
+        want[:k] = orc.scan_u32(want[:k])
+    d = ctx.to_device(a)
+    for k in sizes:
+        gsrb.check(ctx.scan(d, d, k), "scan")
+    ctx.check_status("scan chain")
+    assert np.array_equal(d.download(), want)
+    out = ctx.array(n, np.uint32)
+    with gsrb.CudaGraph(ctx) as g:
+        for k in sizes:
+            gsrb.check(ctx.scan(d, d, k), "scan")
+        gsrb.check(ctx.scan(d, out, n), "scan")
+    d.upload(a)
+    g.launch()
+    ctx.check_status("replay")
+    assert np.array_equal(d.download(), want) and np.array_equal(out.download(), orc.scan_u32(want))
+    d.upload(a)
+    g.launch()
+    ctx.check_status("replay")
+    assert np.array_equal(d.download(), want)
+    g.free()

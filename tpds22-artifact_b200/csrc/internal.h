@@ -26,6 +26,7 @@ struct gsrb_ctx {
   // general scratch (device), grown on demand
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
+  void* stream_words = nullptr;  // scan: state line and tagged tile sums (see scan_stream_kernel)
   // L2 flush buffer
   void* flush = nullptr;
   size_t flush_bytes = 0;

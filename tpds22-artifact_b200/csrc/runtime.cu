@@ -138,7 +138,7 @@ static gsrb_status_t coresident_query(gsrb_ctx* ctx, const void* fn, int block, 
   // raise the kernel's dynamic shared-memory limit to what the device allows
   // next to the kernel's static shared memory (a limit set to this launch's
   // size could be below a later, cached shape's)
-  if (smem > 48 * 1024) {
+  if (smem > 32 * 1024) {  // (static shared memory counts towards the 48 KiB too)
     cudaFuncAttributes fa;
     GSRB_CUDA(cudaFuncGetAttributes(&fa, fn));
     int lim = ctx->max_smem_optin - (int)fa.sharedSizeBytes;
@@ -347,6 +347,12 @@ gsrb_status_t gsrb_ctx_create(int device, gsrb_ctx_t* out) {
   if (e == cudaSuccess) e = cudaMemset(c->flip, 0, fbytes);
   if (e == cudaSuccess) e = cudaMalloc(&c->lf, sizeof(uint32_t) * gsrb::detail::kLfWords);
   if (e == cudaSuccess) e = cudaMemset(c->lf, 0, sizeof(uint32_t) * gsrb::detail::kLfWords);
+  // the streaming scan's state line and words: 16 rounds of one sum (16 bytes) per SM
+  const size_t wbytes = 128 + (size_t)16 * c->num_sms * 16;
+  if (e == cudaSuccess) e = cudaMalloc(&c->stream_words, wbytes);
+  if (e == cudaSuccess) e = cudaMemset(c->stream_words, 0, wbytes);
+  const uint32_t first_tag = 1;  // zeroed words match no round
+  if (e == cudaSuccess) e = cudaMemcpy(c->stream_words, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemset(c->slots, 0, sbytes);
   if (e == cudaSuccess) e = cudaMemset(c->groups, 0, gbytes);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -369,6 +375,7 @@ gsrb_status_t gsrb_ctx_destroy(gsrb_ctx_t c) {
   if (c->flip) cudaFree(c->flip);
   if (c->lf) cudaFree(c->lf);
   if (c->scratch) cudaFree(c->scratch);
+  if (c->stream_words) cudaFree(c->stream_words);
   if (c->flush) cudaFree(c->flush);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;

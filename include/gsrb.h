@@ -158,8 +158,8 @@ gsrb_status_t gsrb_probe_l2_atomics(gsrb_ctx_t ctx, int32_t ctas, int32_t iters,
  * Sum of n int32 into *d_out (int64), one persistent launch: each CTA streams a
  * contiguous chunk through a ring of 32 KiB shared-memory stages filled by
  * cp.async.bulk (cfg->tile = stages, 0 = as many as fit, at most 6), one grid
- * barrier, CTA 0 combines the partials in a fixed order.  cfg == NULL: one
- * 1024-thread CTA per SM.  Replaces reduce_kernel/reduce() of
+ * barrier, one CTA combines the partials in a fixed order.  cfg == NULL:
+ * GSRB_BAR_FANOUT, two 256-thread CTAs per SM.  Replaces reduce_kernel/reduce() of
  * Reduce/reduce_gsrb.cu:289-404 (API Reduce/reduce.cuh:19).  Asynchronous. */
 gsrb_status_t gsrb_reduce_i32(gsrb_ctx_t ctx, const int32_t* d_in, size_t n, int64_t* d_out,
                               const gsrb_cfg_t* cfg);

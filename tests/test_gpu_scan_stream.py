@@ -79,3 +79,22 @@ def test_scan_chain_and_replay(gsrb, ctx, orc):
     ctx.check_status("replay")
     assert np.array_equal(d.download(), want)
     g.free()
+
+
+@pytest.mark.parametrize("n", [0, 1, 5, 4099, 2 * 148 * 4 - 1, 2 * 148 * 4 + 1, 1 << 20, 3_000_001])
+@pytest.mark.parametrize("grid", [0, 1, 2])  # 0: the default call
+def test_reduce_in_order(gsrb, ctx, n, grid):
+    """A reduction reads what the scan before it on the stream wrote, and the
+    one after it may overwrite its input."""
+    c = None if grid == 0 else gsrb.cfg(variant=gsrb.BAR_FANOUT, threads=256, grid_override=grid)
+    a = np.random.default_rng(n).integers(0, 3, max(n, 1)).astype(np.uint32)
+    d, o = ctx.to_device(a), ctx.array(max(n, 1), np.uint32)
+    sums = ctx.array(4, np.int64).zero()
+    want, cur = [], a[:n].astype(np.uint64)
+    for k in range(4):
+        gsrb.check(ctx.scan(d, d, n), "scan")
+        cur = (np.cumsum(cur) - cur) & 0xffffffff if n else cur
+        gsrb.check(ctx.reduce_i32(d, n, sums.at(k), c), "reduce")
+        want.append(int(cur.astype(np.uint32).view(np.int32).astype(np.int64).sum()))
+    ctx.check_status("chain")
+    assert sums.download().tolist() == want

@@ -415,9 +415,11 @@ gsrb_status_t gsrb_probe_gather(gsrb_ctx_t ctx, gsrb_graph_t g, int32_t l1, floa
  * p = 1 - alpha, residuals seeded with (1 - alpha) * alpha * sum 1/outdeg, then
  * rounds of "take the residual, add it to p, push alpha * res / outdeg along
  * every out-edge" over a worklist of vertices whose residual crossed epsilon,
- * until the worklist is empty or max_iters rounds ran.  FP32 atomics in a
- * run-dependent order (as in the reference).  stats->levels = rounds,
- * stats->edges = worklist pushes. */
+ * until the worklist is empty or max_iters rounds ran.  On a symmetric graph the
+ * initial residuals and the rounds with an eighth of the edges or more are
+ * pulled (fixed order, FP64 sums, the residuals below epsilon taken along); the
+ * other rounds push with FP32 atomics in a run-dependent order (as in the
+ * reference).  stats->levels = rounds, stats->edges = worklist pushes. */
 gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t g, float alpha, float epsilon, int32_t max_iters,
                                      float* d_rank, const gsrb_cfg_t* cfg, gsrb_traversal_stats_t* stats);
 

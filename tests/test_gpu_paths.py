@@ -149,3 +149,25 @@ def test_sssp_thin_graphs(gsrb, ctx, orc, thin_graphs, name, delta):
         want = orc.dijkstra(g, src)
         assert np.array_equal(out.download(), want)
         assert st.levels >= 1 and st.edges >= orc.traversed_edges(g, want) and st.delta == delta
+
+
+@pytest.mark.parametrize("name", ["degrees", "bipartite", "grid", "rmat", "tree", "isolated", "path"])
+@pytest.mark.parametrize("shape", ["default", "one_cta"])
+def test_pagerank_residual_rounds(gsrb, ctx, orc, path_graphs, thin_graphs, name, shape):
+    """Pulled and pushed rounds of the residual PageRank against the FP64 fixed
+    point: what is left over is below epsilon a vertex, which the chain of
+    pushes amplifies by at most 1 / (1 - alpha); FP32 sums add 1e-6."""
+    g = path_graphs.get(name) or thin_graphs[name]
+    dg = ctx.graph(g)
+    out = ctx.array(g.nnodes, np.float32)
+    c = None if shape == "default" else gsrb.cfg(variant=gsrb.BAR_FANOUT, threads=128, grid_override=1)
+    ref = orc.pagerank_push(g, 0.85, 200)
+    for eps in (1e-6, 1e-3):
+        rc, st = dg.pagerank_residual(out, 0.85, eps, c=c)
+        gsrb.check(rc, "pagerank_residual")
+        ctx.check_status("pagerank_residual")
+        assert st.levels >= 1
+        assert np.abs(out.download() - ref).sum() <= (eps / 0.15 + 2e-6) * g.nnodes + 2e-6 * ref.sum()
+    rc, st = dg.pagerank_residual(out, 0.85, 1e-9, 3, c)
+    gsrb.check(rc, "pagerank_residual")
+    assert st.levels == 3 or name == "isolated"

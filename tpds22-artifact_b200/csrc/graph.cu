@@ -1709,21 +1709,25 @@ batch_kernel(const BatchDesc* __restrict__ descs, const uint16_t* __restrict__ c
 }
 
 // --------------------------------------------------------------- PageRank ---
+// What a pull pass over a symmetric graph reads besides its input values.
+struct PullArgs {
+  const uint32_t* hubs;   // vertices of degree > kPrHubDegree, ascending
+  const uint32_t* hub_c0; // [nhubs + 1] first chunk of each hub
+  const uint32_t* chunk_hub;  // [nchunks] hub index of each chunk
+  uint32_t nhubs, nchunks;
+  double* part;           // [nchunks] chunk sums
+  uint32_t* hub_done;     // [nhubs] finished chunks (monotonic over passes)
+  unsigned long long* ticket;  // block tickets (monotonic over passes)
+  int32_t gather_l1;      // 1: x/deg gathers through L1 (ld.ca), 0: L2 only (ld.cg)
+};
 struct PrArgs {
   DevCSR g;
   float alpha;
   int32_t iters;
   float* rank;            // output x (FP32)
   float* contrib[2];      // x / deg, double-buffered by iteration parity
-  const uint32_t* hubs;   // vertices of degree > kPrHubDegree, ascending
-  const uint32_t* hub_c0; // [nhubs + 1] first chunk of each hub
-  const uint32_t* chunk_hub;  // [nchunks] hub index of each chunk
-  uint32_t nhubs, nchunks;
-  double* part;           // [nchunks] chunk sums
-  uint32_t* hub_done;     // [nhubs] finished chunks (monotonic over iterations)
-  unsigned long long* ticket;  // block tickets (monotonic over iterations)
+  PullArgs pull;
   uint32_t* out;
-  int32_t gather_l1;      // 1: x/deg gathers through L1 (ld.ca), 0: L2 only (ld.cg)
 };
 
 // One x/deg gather.  Through L1 the hubs' entries (read by many rows of a
@@ -1772,16 +1776,130 @@ __device__ __forceinline__ double warp_gather_sum(const uint32_t* __restrict__ d
   return s;
 }
 
-// Pull PageRank, one grid barrier per iteration.
+// One pull pass: done(v, degree, sum of cin over v's row) once for every vertex,
+// by one lane; pass number `it` of the launch, warp gw of nw.
 //  * Hubs (degree > kPrHubDegree) are cut into chunks of kPrChunk edges; a warp
 //    sums a chunk, stores it, and bumps the hub's counter (acq_rel); the warp
-//    that finishes a hub's last chunk adds the chunk sums in chunk order and
-//    writes the hub's rank and contribution.
+//    that finishes a hub's last chunk adds the chunk sums in chunk order.
 //  * Every other vertex: a warp takes 32 consecutive vertices and walks their
 //    concatenated edge lists 32 edges per round (coalesced dst loads); each
 //    lane finds the owner of its edge by a binary search over the lanes'
 //    exclusive degree prefix, and a segmented shuffle scan hands each owner its
 //    segment's sum.  Per-vertex FP64 sums in a fixed order.
+template <class F>
+__device__ __forceinline__ void pull_pass(const DevCSR& g, const PullArgs& a, const float* cin, uint32_t it, uint32_t gw,
+                                          uint32_t nw, F& done) {
+  const uint32_t lane = lane_id();
+  // ---- hub chunks
+  for (uint32_t c = gw; c < a.nchunks; c += nw) {
+    const uint32_t k = __ldg(a.chunk_hub + c);
+    const uint32_t u = __ldg(a.hubs + k);
+    const uint32_t c0 = __ldg(a.hub_c0 + k), c1 = __ldg(a.hub_c0 + k + 1);
+    const uint32_t ub = __ldg(g.row + u), ue = __ldg(g.row + u + 1);
+    const uint32_t j0 = ub + (c - c0) * kPrChunk;
+    const uint32_t j1 = min(ue, j0 + kPrChunk);
+    const double t = warp_gather_sum(g.dst, cin, j0, j1, lane, a.gather_l1);
+    uint32_t last = 0;
+    if (lane == 0) {
+      a.part[c] = t;
+      const uint32_t target = (c1 - c0) * (it + 1u);
+      last = gsrb::ptx::atom_add_acq_rel_gpu(a.hub_done + k, 1u) + 1u == target;
+    }
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (last) {
+      // fixed order: lane-strided chunk sums, then the same butterfly
+      double s = 0.0;
+      for (uint32_t i = c0 + lane; i < c1; i += 32) s += __ldcg(a.part + i);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+      if (lane == 0) done(u, ue - ub, s);
+    }
+  }
+  // ---- everything else: blocks of 32 consecutive vertices, taken by warps
+  // from a ticket counter (block sizes vary by orders of magnitude)
+  const uint32_t nblocks = (g.n + 31u) >> 5;
+  const unsigned long long tbase = (unsigned long long)it * (nblocks + nw);
+  for (;;) {
+    unsigned long long t = 0;
+    if (lane == 0) t = atomicAdd(a.ticket, 1ull);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    const unsigned long long blk = t - tbase;
+    if (blk >= nblocks) break;  // every warp draws exactly one ticket past the end
+    const uint32_t v = (uint32_t)blk * 32u + lane;
+    uint32_t b = 0, d = 0;
+    bool mine = false;
+    if (v < g.n) {
+      b = __ldg(g.row + v);
+      const uint32_t dd = __ldg(g.row + v + 1) - b;
+      mine = dd <= kPrHubDegree;
+      d = mine ? dd : 0u;
+    }
+    uint32_t inc = d;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
+      if ((int)lane >= o) inc += y;
+    }
+    const uint32_t excl = inc - d;
+    const uint32_t E = __shfl_sync(0xffffffffu, inc, 31);
+    double acc = 0.0;
+    // kRounds rounds of 32 edges per step: all gathers of a step in flight together
+    constexpr int kRounds = 4;
+    for (uint32_t f0 = 0; f0 < E; f0 += 32u * kRounds) {
+      uint32_t own[kRounds], nbr[kRounds];
+      double val[kRounds];
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        const uint32_t f = f0 + 32u * r + lane;
+        // owner = the last lane whose exclusive prefix is <= f; the search
+        // carries that prefix along (lane 0's is 0), so it costs no shuffle
+        uint32_t lo = 0, oe = 0;
+#pragma unroll
+        for (uint32_t step = 16; step > 0; step >>= 1) {
+          const uint32_t x = __shfl_sync(0xffffffffu, excl, lo + step);
+          if (x <= f) {
+            lo += step;
+            oe = x;
+          }
+        }
+        // the lane (of this round) where the owner's segment begins: the
+        // segmented scan below compares lanes against it instead of
+        // shuffling owners
+        own[r] = oe > f0 + 32u * r ? oe - (f0 + 32u * r) : 0u;
+        const uint32_t ob = __shfl_sync(0xffffffffu, b, lo);
+        nbr[r] = f < E ? __ldg(g.dst + ob + (f - oe)) : 0u;
+      }
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        const uint32_t f = f0 + 32u * r + lane;
+        val[r] = f < E ? (double)pr_gather(cin, nbr[r], a.gather_l1) : 0.0;
+      }
+#pragma unroll
+      for (int r = 0; r < kRounds; ++r) {
+        const uint32_t rb = f0 + 32u * r;
+        if (rb >= E) break;  // warp-uniform
+        // segmented inclusive scan: lane l - o belongs to the same owner
+        // as lane l exactly when l - o is not before the owner's first lane
+        double x = val[r];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double y = __shfl_up_sync(0xffffffffu, x, o);
+          if ((int)lane - o >= (int)own[r]) x += y;
+        }
+        // this lane's vertex: its segment in this round ends at flat index
+        // min(excl + d, rb + 32, E) - 1
+        const uint32_t seg_b = excl > rb ? excl : rb;
+        const uint32_t seg_e = min(min(excl + d, rb + 32u), E);
+        const uint32_t endl = seg_e > seg_b ? seg_e - 1u - rb : 0u;
+        const double t2 = __shfl_sync(0xffffffffu, x, endl);
+        if (seg_e > seg_b) acc += t2;
+      }
+    }
+    if (mine) done(v, d, acc);
+  }
+}
+
+// Pull PageRank, one grid barrier per iteration (see pull_pass).
 template <int V>
 __global__ void __launch_bounds__(1024)
 pagerank_kernel(gsrb::GridBarrier gb, PrArgs a) {
@@ -1798,127 +1916,17 @@ pagerank_kernel(gsrb::GridBarrier gb, PrArgs a) {
     a.contrib[0][v] = d ? base / (float)d : 0.f;
   }
   ok = bar.sync() && ok;
-  const uint32_t lane = lane_id();
   const uint32_t gw = tid >> 5, nw = nthreads >> 5;
   int32_t it = 0;
   for (; ok && it < a.iters; ++it) {
     const float* cin = a.contrib[it & 1];
     float* cout = a.contrib[(it + 1) & 1];
-    // ---- hub chunks
-    for (uint32_t c = gw; c < a.nchunks; c += nw) {
-      const uint32_t k = __ldg(a.chunk_hub + c);
-      const uint32_t u = __ldg(a.hubs + k);
-      const uint32_t c0 = __ldg(a.hub_c0 + k), c1 = __ldg(a.hub_c0 + k + 1);
-      const uint32_t ub = __ldg(g.row + u), ue = __ldg(g.row + u + 1);
-      const uint32_t j0 = ub + (c - c0) * kPrChunk;
-      const uint32_t j1 = min(ue, j0 + kPrChunk);
-      const double t = warp_gather_sum(g.dst, cin, j0, j1, lane, a.gather_l1);
-      uint32_t last = 0;
-      if (lane == 0) {
-        a.part[c] = t;
-        const uint32_t target = (c1 - c0) * (uint32_t)(it + 1);
-        last = gsrb::ptx::atom_add_acq_rel_gpu(a.hub_done + k, 1u) + 1u == target;
-      }
-      last = __shfl_sync(0xffffffffu, last, 0);
-      if (last) {
-        // fixed order: lane-strided chunk sums, then the same butterfly
-        double s = 0.0;
-        for (uint32_t i = c0 + lane; i < c1; i += 32) s += __ldcg(a.part + i);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) {
-          const float x = (float)((double)base + (double)a.alpha * s);
-          a.rank[u] = x;
-          cout[u] = x / (float)(ue - ub);
-        }
-      }
-    }
-    // ---- everything else: blocks of 32 consecutive vertices, taken by warps
-    // from a ticket counter (block sizes vary by orders of magnitude)
-    const uint32_t nblocks = (g.n + 31u) >> 5;
-    const unsigned long long tbase = (unsigned long long)it * (nblocks + nw);
-    for (;;) {
-      unsigned long long t = 0;
-      if (lane == 0) t = atomicAdd(a.ticket, 1ull);
-      t = __shfl_sync(0xffffffffu, t, 0);
-      const unsigned long long blk = t - tbase;
-      if (blk >= nblocks) break;  // every warp draws exactly one ticket past the end
-      const uint32_t v = (uint32_t)blk * 32u + lane;
-      uint32_t b = 0, d = 0;
-      bool mine = false;
-      if (v < g.n) {
-        b = __ldg(g.row + v);
-        const uint32_t dd = __ldg(g.row + v + 1) - b;
-        mine = dd <= kPrHubDegree;
-        d = mine ? dd : 0u;
-      }
-      uint32_t inc = d;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, inc, o);
-        if ((int)lane >= o) inc += y;
-      }
-      const uint32_t excl = inc - d;
-      const uint32_t E = __shfl_sync(0xffffffffu, inc, 31);
-      double acc = 0.0;
-      // kRounds rounds of 32 edges per step: all gathers of a step in flight together
-      constexpr int kRounds = 4;
-      for (uint32_t f0 = 0; f0 < E; f0 += 32u * kRounds) {
-        uint32_t own[kRounds], nbr[kRounds];
-        double val[kRounds];
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r) {
-          const uint32_t f = f0 + 32u * r + lane;
-          // owner = the last lane whose exclusive prefix is <= f; the search
-          // carries that prefix along (lane 0's is 0), so it costs no shuffle
-          uint32_t lo = 0, oe = 0;
-#pragma unroll
-          for (uint32_t step = 16; step > 0; step >>= 1) {
-            const uint32_t x = __shfl_sync(0xffffffffu, excl, lo + step);
-            if (x <= f) {
-              lo += step;
-              oe = x;
-            }
-          }
-          // the lane (of this round) where the owner's segment begins: the
-          // segmented scan below compares lanes against it instead of
-          // shuffling owners
-          own[r] = oe > f0 + 32u * r ? oe - (f0 + 32u * r) : 0u;
-          const uint32_t ob = __shfl_sync(0xffffffffu, b, lo);
-          nbr[r] = f < E ? __ldg(g.dst + ob + (f - oe)) : 0u;
-        }
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r) {
-          const uint32_t f = f0 + 32u * r + lane;
-          val[r] = f < E ? (double)pr_gather(cin, nbr[r], a.gather_l1) : 0.0;
-        }
-#pragma unroll
-        for (int r = 0; r < kRounds; ++r) {
-          const uint32_t rb = f0 + 32u * r;
-          if (rb >= E) break;  // warp-uniform
-          // segmented inclusive scan: lane l - o belongs to the same owner
-          // as lane l exactly when l - o is not before the owner's first lane
-          double x = val[r];
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const double y = __shfl_up_sync(0xffffffffu, x, o);
-            if ((int)lane - o >= (int)own[r]) x += y;
-          }
-          // this lane's vertex: its segment in this round ends at flat index
-          // min(excl + d, rb + 32, E) - 1
-          const uint32_t seg_b = excl > rb ? excl : rb;
-          const uint32_t seg_e = min(min(excl + d, rb + 32u), E);
-          const uint32_t endl = seg_e > seg_b ? seg_e - 1u - rb : 0u;
-          const double t2 = __shfl_sync(0xffffffffu, x, endl);
-          if (seg_e > seg_b) acc += t2;
-        }
-      }
-      if (mine) {
-        const float x = (float)((double)base + (double)a.alpha * acc);
-        a.rank[v] = x;
-        cout[v] = d ? x / (float)d : 0.f;
-      }
-    }
+    auto done = [&](uint32_t v, uint32_t d, double sum) {
+      const float x = (float)((double)base + (double)a.alpha * sum);
+      a.rank[v] = x;
+      cout[v] = d ? x / (float)d : 0.f;
+    };
+    pull_pass(g, a.pull, cin, (uint32_t)it, gw, nw, done);
     ok = bar.sync();
   }
   if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -1955,7 +1963,16 @@ struct PrrArgs {
   uint32_t* overflow;
   uint32_t* out;        // [0] rounds, [1] worklist pushes (low 32 bits), [3] failure
   unsigned long long* out_edges;
+  PullArgs pull;
+  bool symmetric;       // rows are also in-edge lists: rounds with many edges may pull
 };
+
+// A round whose worklist holds at least 1 / kPrrDense of the edges is pulled on
+// a symmetric graph: the same round (every vertex of the list takes its
+// residual, every neighbour receives its shares) without an atomic per edge.
+// R-MAT-20: a pull round takes 0.15 ms whatever the list, a push round about
+// 1 ms for all the edges.
+constexpr unsigned long long kPrrDense = 8;
 
 // Vertices of the regular queue with more edges than this are pushed by their
 // whole CTA (after the CTA's warps have walked their queue groups), so that one
@@ -1972,7 +1989,8 @@ struct PrrSink {
   unsigned long long* n_reg;
   unsigned long long* n_big;
   uint32_t stamp;  // a vertex enters the next worklist at most once per round
-  WarpRes* res;    // the warp's worklist reservation (chunk 0: direct appends)
+  IdStage* stage;  // the CTA's worklist entries
+  WarpRes* res;    // the warp's worklist reservation (past the stage)
 };
 
 // Push residual along four edges per lane at once: edge r of the lane is j[r]
@@ -1982,20 +2000,21 @@ struct PrrSink {
 // r[dst] += alpha * res / outdeg, pushed when it crosses epsilon).
 // Warp-synchronous.
 __device__ __forceinline__ void prr_push4e(const PrrArgs& a, const float* upd, const uint32_t* j, uint32_t act,
-                                           const PrrSink& s, unsigned long long& pushes) {
+                                           const PrrSink& s, unsigned long long& pushes,
+                                           unsigned long long& medges) {
   const DevCSR& g = a.g;
   uint32_t w[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) w[r] = ((act >> r) & 1u) ? __ldg(g.dst + j[r]) : 0u;
-  bool cross[4];
+  float prev[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
-    cross[r] = false;
-    if ((act >> r) & 1u) {
-      const float prev = atomicAdd(a.r + w[r], upd[r]);
-      cross[r] = prev + upd[r] > a.eps && prev < a.eps;
-    }
+    prev[r] = a.eps;
+    if ((act >> r) & 1u) prev[r] = atomicAdd(a.r + w[r], upd[r]);
   }
+  bool cross[4];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) cross[r] = ((act >> r) & 1u) && prev[r] + upd[r] > a.eps && prev[r] < a.eps;
   // the row range of a candidate goes out with its stamp exchange (one round
   // trip instead of two; unused when the exchange finds it already queued)
   uint32_t rb[4], re[4];
@@ -2005,7 +2024,11 @@ __device__ __forceinline__ void prr_push4e(const PrrArgs& a, const float* upd, c
     re[r] = cross[r] ? __ldg(g.row + w[r] + 1) : 0u;
   }
 #pragma unroll
-  for (int r = 0; r < 4; ++r) cross[r] = cross[r] && atomicExch(a.mark + w[r], s.stamp) != s.stamp;
+  for (int r = 0; r < 4; ++r) {
+    uint32_t st = s.stamp;
+    if (cross[r]) st = atomicExch(a.mark + w[r], s.stamp);
+    cross[r] = st != s.stamp;
+  }
   bool reg[4], big[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
@@ -2013,25 +2036,10 @@ __device__ __forceinline__ void prr_push4e(const PrrArgs& a, const float* upd, c
     reg[r] = cross[r] && d <= kBigDegree;
     big[r] = cross[r] && d > kBigDegree;
     pushes += cross[r] ? 1u : 0u;
+    medges += d;
   }
-  if (s.res->chunk) warp_append_res<4>(reg, w, s.qout, s.n_reg, 2u * g.n, a.overflow, *s.res, kHole);
-  else warp_append_k<4>(reg, w, s.qout, s.n_reg, g.n, a.overflow);
+  stage_append<4>(reg, w, *s.stage, s.qout, s.n_reg, g.n, 2u * g.n, a.overflow, *s.res, kHole);
   warp_append_k<4>(big, w, s.hout, s.n_big, g.n, a.overflow);
-}
-
-// The same from one vertex: edge r is jbase + r * stride while below jend.
-__device__ __forceinline__ void prr_push4(const PrrArgs& a, float upd, uint32_t jbase, uint32_t stride, uint32_t jend,
-                                          const PrrSink& s, unsigned long long& pushes) {
-  float u4[4];
-  uint32_t j[4];
-  uint32_t act = 0;
-#pragma unroll
-  for (int r = 0; r < 4; ++r) {
-    u4[r] = upd;
-    j[r] = jbase + (uint32_t)r * stride;
-    if (j[r] < jend) act |= 1u << r;
-  }
-  prr_push4e(a, u4, j, act, s, pushes);
 }
 
 // A list of vertices pushed edge-balanced: edge prefix p[0..cnt], first edges
@@ -2039,7 +2047,8 @@ __device__ __forceinline__ void prr_push4(const PrrArgs& a, float upd, uint32_t 
 // (x & ~31) + lane + k * nthr, four per step.  Warp-synchronous loops.
 __device__ __forceinline__ void prr_push_list(const PrrArgs& a, const uint32_t* p, const uint32_t* b,
                                               const int32_t* d, uint32_t cnt, uint32_t x, uint32_t nthr,
-                                              const PrrSink& s, unsigned long long& pushes) {
+                                              const PrrSink& s, unsigned long long& pushes,
+                                              unsigned long long& medges) {
   const uint32_t total = p[cnt];
   for (uint32_t t0 = (x & ~31u) + lane_id(); t0 - lane_id() < total; t0 += 4u * nthr) {
     float upd[4];
@@ -2057,7 +2066,7 @@ __device__ __forceinline__ void prr_push_list(const PrrArgs& a, const uint32_t* 
         act |= 1u << r;
       }
     }
-    prr_push4e(a, upd, j, act, s, pushes);
+    prr_push4e(a, upd, j, act, s, pushes, medges);
   }
 }
 
@@ -2071,6 +2080,8 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
   const Team team{blockIdx.x, gridDim.x};
   const uint32_t tid = team.tid(), nthreads = team.nthreads();
   const uint32_t lane = lane_id();
+  __shared__ IdStage s_stage;
+  if (threadIdx.x == 0) stage_reset(s_stage);
   // init_1
   for (uint32_t v = tid; v < g.n; v += nthreads) {
     a.p[v] = 1.f - a.alpha;
@@ -2078,25 +2089,40 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
     a.mark[v] = 0;
   }
   if (tid == 0)
-    for (int k = 0; k < 3; ++k) a.cnt[k].n_reg = a.cnt[k].n_big = a.cnt[k].m_next = 0;
+    for (int k = 0; k < 3; ++k) a.cnt[k].n_reg = a.cnt[k].n_real = a.cnt[k].n_big = a.cnt[k].m_next = 0;
   ok = bar.sync() && ok;
-  for (uint32_t gwarp = tid >> 5; gwarp * 32u < g.n; gwarp += nthreads >> 5) {
-    const uint32_t u = gwarp * 32u + lane;
-    uint32_t b = 0, e = 0;
-    if (u < g.n) {
-      b = __ldg(g.row + u);
-      e = __ldg(g.row + u + 1);
+  bool dense = a.symmetric;
+  uint32_t pulls = 0;
+  if (dense) {
+    // the neighbours' 1 / outdeg, pulled (an atomic per edge took about 1 ms on R-MAT-20)
+    for (uint32_t v = tid; v < g.n; v += nthreads) {
+      const uint32_t d = __ldg(g.row + v + 1) - __ldg(g.row + v);
+      a.hub_upd[v] = d ? 1.f / (float)d : 0.f;
     }
-    const float upd = e > b ? 1.f / (float)(e - b) : 0.f;
-    // warp-strided edges of the 32 vertices, one vertex at a time
-    for (int src = 0; src < 32; ++src) {
-      const uint32_t bb = __shfl_sync(0xffffffffu, b, src), ee = __shfl_sync(0xffffffffu, e, src);
-      const float uu = __shfl_sync(0xffffffffu, upd, src);
-      for (uint32_t j = bb + lane; j < ee; j += 32) atomicAdd(a.r + __ldg(g.dst + j), uu);
+    ok = bar.sync() && ok;
+    auto done = [&](uint32_t v, uint32_t, double sum) { a.r[v] = (float)sum; };
+    if (ok) pull_pass(g, a.pull, a.hub_upd, pulls, tid >> 5, nthreads >> 5, done);
+    ++pulls;
+  } else {
+    for (uint32_t gwarp = tid >> 5; gwarp * 32u < g.n; gwarp += nthreads >> 5) {
+      const uint32_t u = gwarp * 32u + lane;
+      uint32_t b = 0, e = 0;
+      if (u < g.n) {
+        b = __ldg(g.row + u);
+        e = __ldg(g.row + u + 1);
+      }
+      const float upd = e > b ? 1.f / (float)(e - b) : 0.f;
+      // warp-strided edges of the 32 vertices, one vertex at a time
+      for (int src = 0; src < 32; ++src) {
+        const uint32_t bb = __shfl_sync(0xffffffffu, b, src), ee = __shfl_sync(0xffffffffu, e, src);
+        const float uu = __shfl_sync(0xffffffffu, upd, src);
+        for (uint32_t j = bb + lane; j < ee; j += 32) atomicAdd(a.r + __ldg(g.dst + j), uu);
+      }
     }
   }
   ok = bar.sync() && ok;
-  // init_2: scale, every vertex enters the worklist (hubs to the hub queue)
+  // init_2: scale, every vertex enters the worklist (hubs to the hub queue; a
+  // pulled first round needs no list)
   for (uint32_t base = (tid >> 5) * 32u; base < g.n; base += nthreads) {
     const uint32_t v = base + lane;
     bool reg = false, big = false;
@@ -2106,25 +2132,104 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
       big = d > kBigDegree;
       reg = !big;
     }
-    warp_append(reg, v, a.q[0], &a.cnt[0].n_reg, g.n, a.overflow);
-    warp_append(big, v, a.hq[0], &a.cnt[0].n_big, g.n, a.overflow);
+    if (!dense) {
+      warp_append(reg, v, a.q[0], &a.cnt[0].n_reg, g.n, a.overflow);
+      warp_append(big, v, a.hq[0], &a.cnt[0].n_big, g.n, a.overflow);
+    }
   }
   ok = bar.sync() && ok;
+  __shared__ unsigned long long s_edges, s_active;
   uint32_t round = 0;
   unsigned long long pushes = 0;
   for (; ok && round < (uint32_t)a.max_iters; ++round) {
+    LevelCounters* c = &a.cnt[(round + 1) % 3];
+    uint32_t* qout = a.q[(round + 1) & 1];
+    uint32_t* hout = a.hq[(round + 1) & 1];
+    if (threadIdx.x == 0) s_edges = s_active = 0;
+    if (dense) {
+      // the list is the vertices above epsilon (in the first round all of
+      // them); a pull costs the same with the rest's residuals, so those are
+      // taken along and less is left over at the end
+      float* share = a.hub_upd;
+      for (uint32_t v = tid; v < g.n; v += nthreads) {
+        const float res = a.r[v];
+        float x = 0.f;
+        if (res != 0.f) {
+          a.r[v] = 0.f;
+          a.p[v] += res;
+          const uint32_t d = __ldg(g.row + v + 1) - __ldg(g.row + v);
+          x = d ? res * a.alpha / (float)d : 0.f;
+        }
+        share[v] = x;
+      }
+      if (tid == 0) {
+        // counters of the round after next, last read before the barrier that ended the round before
+        LevelCounters* z = &a.cnt[(round + 2) % 3];
+        z->n_reg = z->n_big = z->n_real = z->m_next = 0;
+      }
+      ok = bar.sync();
+      if (!ok) break;
+      unsigned long long medges = 0;
+      uint32_t nact = 0;
+      auto done = [&](uint32_t v, uint32_t d, double sum) {
+        const float r = a.r[v] + (float)sum;
+        a.r[v] = r;
+        if (r > a.eps) {
+          ++nact;
+          medges += d;
+        }
+      };
+      pull_pass(g, a.pull, share, pulls, tid >> 5, nthreads >> 5, done);
+      ++pulls;
+      medges = warp_sum_u64(medges);
+      const uint32_t wact = __reduce_add_sync(0xffffffffu, nact);
+      if (lane == 0 && wact) {
+        atomicAdd(&s_edges, medges);
+        atomicAdd(&s_active, (unsigned long long)wact);
+      }
+      __syncthreads();
+      if (threadIdx.x == 0 && s_active) {
+        atomicAdd(&c->m_next, s_edges);
+        atomicAdd(&c->n_real, s_active);
+      }
+      ok = bar.sync();
+      if (!ok) break;
+      const unsigned long long act = __ldcg(&c->n_real), me = __ldcg(&c->m_next);
+      if (tid == 0) pushes += act;
+      if (act == 0) {
+        ++round;
+        break;
+      }
+      dense = me * kPrrDense >= g.m;
+      if (!dense) {
+        // the rounds that follow push: make the list
+        for (uint32_t base = (tid >> 5) * 32u; base < g.n; base += nthreads) {
+          const uint32_t v = base + lane;
+          bool in = v < g.n && a.r[v] > a.eps;
+          uint32_t d = 0;
+          if (in) d = __ldg(g.row + v + 1) - __ldg(g.row + v);
+          const bool reg[1] = {in && d <= kBigDegree};
+          const uint32_t vv[1] = {v};
+          WarpRes none{0ull, 0u, 0u};
+          stage_append<1>(reg, vv, s_stage, qout, &c->n_reg, g.n, 2u * g.n, a.overflow, none, kHole);
+          warp_append(in && d > kBigDegree, v, hout, &c->n_big, g.n, a.overflow);
+        }
+        stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
+        ok = bar.sync();
+        if (!ok) break;
+      }
+      continue;
+    }
     const uint32_t nreg = (uint32_t)__ldcg(&a.cnt[round % 3].n_reg);
     const uint32_t nbig = (uint32_t)__ldcg(&a.cnt[round % 3].n_big);
     if (nreg + nbig == 0) break;
     if (tid == 0) {
-      a.cnt[(round + 2) % 3].n_reg = 0;
-      a.cnt[(round + 2) % 3].n_big = 0;
+      LevelCounters* z = &a.cnt[(round + 2) % 3];
+      z->n_reg = z->n_big = z->n_real = z->m_next = 0;
     }
     const uint32_t* qin = a.q[round & 1];
     const uint32_t* hin = a.hq[round & 1];
-    uint32_t* qout = a.q[(round + 1) & 1];
-    uint32_t* hout = a.hq[(round + 1) & 1];
-    LevelCounters* c = &a.cnt[(round + 1) % 3];
+    unsigned long long medges = 0;  // edges of the vertices this thread queues
     // a vertex whose residual crosses epsilon twice in one round (its own
     // exchange in this round restarted it from 0) enters the next list once
     const uint32_t stamp = round + 2u;
@@ -2136,11 +2241,12 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
       warp_append(cross && d <= kBigDegree, w, qout, &c->n_reg, 2u * g.n, a.overflow);
       warp_append(cross && d > kBigDegree, w, hout, &c->n_big, g.n, a.overflow);
       pushes += cross ? 1u : 0u;
+      medges += d;
     };
     // worklist reservations in chunks of 64 slots when the queue (2n slots)
     // can hold the holes of every warp (see WarpRes)
     WarpRes wres{0ull, 0u, 63ull * (nthreads >> 5) <= g.n ? 64u : 0u};
-    const PrrSink sink{qout, hout, &c->n_reg, &c->n_big, stamp, &wres};
+    const PrrSink sink{qout, hout, &c->n_reg, &c->n_big, stamp, &s_stage, &wres};
     ListSmem& L_ = list_smem();
     // builds an edge-balanced list from vertex ids and their updates (CTA-wide)
     auto build_list = [&](auto id_of, auto upd_of, uint32_t cnt) {
@@ -2176,7 +2282,7 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
       if (nbig <= kHubList) {
         build_list([&](uint32_t i) { return __ldcg(hin + i); },
                    [&](uint32_t, uint32_t u) { return __ldcg(a.hub_upd + u); }, nbig);
-        prr_push_list(a, L_.p, L_.b, L_.d, nbig, tid, nthreads, sink, pushes);
+        prr_push_list(a, L_.p, L_.b, L_.d, nbig, tid, nthreads, sink, pushes, medges);
         __syncthreads();
       } else {
         auto hub_edge = [&](uint32_t u, uint32_t j, bool active) {
@@ -2194,56 +2300,58 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
       }
     }
     // regular worklist: a lane per vertex exchanges its residual once; edges
-    // of degree > kCtaDegree vertices go to the CTA's edge-balanced list,
-    // degree > kWarpDegree across the warp, the rest per lane, four edges per
-    // lane in flight
+    // of degree > kCtaDegree vertices go to the CTA's edge-balanced list, the
+    // rest edge-balanced over the warp, four edges per lane in flight
     __shared__ uint32_t s_cta_u[kCtaListCap];
     __shared__ float s_cta_upd[kCtaListCap];
     __shared__ uint32_t s_ncta;
     if (threadIdx.x == 0) s_ncta = 0;
     __syncthreads();
-    for (uint32_t base = (tid >> 5) * 32u; base < nreg; base += nthreads) {
+    const uint32_t nwarps = nthreads >> 5, gsz = group_size_of(nreg, nwarps);
+    for (uint32_t base = spread_warp(team) * gsz; base < nreg; base += nwarps * gsz) {
       const uint32_t i = base + lane;
+      const bool in = lane < gsz && i < nreg;
       uint32_t u = 0, b = 0, e = 0;
       float upd = 0.f;
-      if (i < nreg) u = __ldcg(qin + i);
-      if (i < nreg && u != kHole) {
+      if (in) u = __ldcg(qin + i);
+      if (in && u != kHole) {
         b = __ldg(g.row + u);
         e = __ldg(g.row + u + 1);
         const float res = atomicExch(a.r + u, 0.f);
         atomicAdd(a.p + u, res);
         upd = e > b ? res * a.alpha / (float)(e - b) : 0.f;
       }
-      const uint32_t deg = e - b;
-      bool warp_tier = deg > kWarpDegree;
+      uint32_t deg = e - b;
       if (deg > kCtaDegree) {
         const uint32_t slot = atomicAdd(&s_ncta, 1u);
         if (slot < kCtaListCap) {
           s_cta_u[slot] = u;
           s_cta_upd[slot] = upd;
-          warp_tier = false;
+          deg = 0;
         }
       }
-      uint32_t coop = __ballot_sync(0xffffffffu, warp_tier);
-      while (coop) {
-        const int src = __ffs(coop) - 1;
-        coop &= coop - 1;
-        const uint32_t bb = __shfl_sync(0xffffffffu, b, src), ee = __shfl_sync(0xffffffffu, e, src);
-        const float uu = __shfl_sync(0xffffffffu, upd, src);
-        for (uint32_t j0 = bb; j0 < ee; j0 += 128) prr_push4(a, uu, j0 + lane, 32u, ee, sink, pushes);
-      }
-      const uint32_t mine = deg <= kWarpDegree ? deg : 0u;
-      const uint32_t kmax = warp_max_u32(mine);
-      for (uint32_t k0 = 0; k0 < kmax; k0 += 4) prr_push4(a, upd, b + k0, 1u, b + mine, sink, pushes);
+      auto step = [&](const uint32_t* j, const uint32_t* own, uint32_t act) {
+        float u4[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) u4[r] = __shfl_sync(0xffffffffu, upd, own[r]);
+        prr_push4e(a, u4, j, act, sink, pushes, medges);
+      };
+      walk_group(b, deg, step);
     }
     __syncthreads();
     const uint32_t ncta = min(s_ncta, kCtaListCap);
     if (ncta) {
       build_list([&](uint32_t i) { return s_cta_u[i]; }, [&](uint32_t i, uint32_t) { return s_cta_upd[i]; }, ncta);
-      prr_push_list(a, L_.p, L_.b, L_.d, ncta, threadIdx.x, blockDim.x, sink, pushes);
+      prr_push_list(a, L_.p, L_.b, L_.d, ncta, threadIdx.x, blockDim.x, sink, pushes, medges);
     }
     warp_res_close(qout, 2u * g.n, wres, kHole);
+    medges = warp_sum_u64(medges);
+    if (lane == 0 && medges) atomicAdd(&s_edges, medges);
+    stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
+    if (threadIdx.x == 0 && s_edges) atomicAdd(&c->m_next, s_edges);
     ok = bar.sync();
+    if (!ok) break;
+    dense = a.symmetric && __ldcg(&c->m_next) * kPrrDense >= g.m;
   }
   const unsigned long long ws = warp_sum_u64(pushes);
   if (lane == 0 && ws) atomicAdd(a.out_edges, ws);
@@ -2569,6 +2677,20 @@ gsrb_cfg_t graph_cfg(gsrb_ctx* ctx, const gsrb_cfg_t* in) {
     c.cluster = 2;
   }
   return c;
+}
+
+PullArgs pull_args(const gsrb_graph* G, const gsrb_cfg_t& c) {
+  PullArgs a;
+  a.hubs = G->hubs;
+  a.hub_c0 = G->hub_c0;
+  a.chunk_hub = G->chunk_hub;
+  a.nhubs = G->nhubs;
+  a.nchunks = G->nchunks;
+  a.part = G->hub_part;
+  a.hub_done = G->hub_done;
+  a.ticket = reinterpret_cast<unsigned long long*>(G->flags + 24);
+  a.gather_l1 = c.form == GSRB_FORM_L2 ? 0 : 1;
+  return a;
 }
 
 // CTAs of the cluster that runs thin steps: 16, 8 where 16 cannot be placed,
@@ -3053,16 +3175,8 @@ gsrb_status_t gsrb_pagerank(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha, int32_t
   a.rank = d_rank;
   a.contrib[0] = G->contrib[0];
   a.contrib[1] = G->contrib[1];
-  a.hubs = G->hubs;
-  a.hub_c0 = G->hub_c0;
-  a.chunk_hub = G->chunk_hub;
-  a.nhubs = G->nhubs;
-  a.nchunks = G->nchunks;
-  a.part = G->hub_part;
-  a.hub_done = G->hub_done;
-  a.ticket = reinterpret_cast<unsigned long long*>(G->flags + 24);
+  a.pull = pull_args(G, c);
   a.out = G->flags + 4;
-  a.gather_l1 = c.form == GSRB_FORM_L2 ? 0 : 1;
   G->last_delta = 0;
   std::lock_guard<std::mutex> g(ctx->mu);
   GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
@@ -3096,6 +3210,8 @@ gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha
   a.eps = epsilon;
   a.max_iters = max_iters;
   a.p = d_rank;
+  a.pull = pull_args(G, c);
+  a.symmetric = G->symmetric;
   a.r = G->contrib[0];
   a.hub_upd = G->contrib[1];
   a.mark = G->mark;
@@ -3110,6 +3226,7 @@ gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha
   G->last_delta = 0;
   std::lock_guard<std::mutex> g(ctx->mu);
   GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
+  if (G->nhubs) GSRB_CUDA(cudaMemsetAsync(G->hub_done, 0, sizeof(uint32_t) * G->nhubs, ctx->stream));
   gsrb::GridBarrier gb = make_barrier(ctx, c, 0, (uint32_t)grid, 0, 0);
   void* args[] = {&gb, &a};
   if (!ctx->events[62]) GSRB_CUDA(cudaEventCreate(&ctx->events[62]));

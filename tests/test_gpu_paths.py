@@ -171,3 +171,19 @@ def test_pagerank_residual_rounds(gsrb, ctx, orc, path_graphs, thin_graphs, name
     rc, st = dg.pagerank_residual(out, 0.85, 1e-9, 3, c)
     gsrb.check(rc, "pagerank_residual")
     assert st.levels == 3 or name == "isolated"
+
+
+@pytest.mark.parametrize("name", ["degrees", "bipartite", "grid", "rmat"])
+@pytest.mark.parametrize("mode", [1, 3])  # heuristic, pull every level after the first
+def test_bfs_pull_rows(gsrb, ctx, orc, path_graphs, name, mode):
+    """Pull levels over rows at the edges of the lane / warp split (4, 32, 128 edges)."""
+    g = path_graphs[name]
+    dg = ctx.graph(g)
+    out = ctx.array(g.nnodes, np.int32)
+    for src in (0, 7, g.nnodes - 1):
+        for c in (None, gsrb.cfg(variant=gsrb.BAR_FANOUT, threads=64, grid_override=3)):
+            rc, st = dg.bfs(src, out, mode, c)
+            gsrb.check(rc, "bfs")
+            want = orc.bfs(g, src)
+            assert np.array_equal(out.download(), want)
+            assert st.edges == orc.traversed_edges(g, want)

@@ -61,8 +61,9 @@ constexpr uint32_t kThinDegree = 8;           // graphs below this mean degree s
 constexpr uint32_t kClQueue = 4096;           // entries per CTA and parity
 constexpr uint32_t kClMaxFrontier = 16384;    // larger levels go to the grid: past this 16 SMs' gathers
 constexpr uint32_t kClMaxEdges = 65536;       // (one a cycle and SM) cost more than a grid level
-constexpr uint32_t kClEnterFrontier = 2048;   // and come back below these
-constexpr unsigned long long kClEnterEdges = 8192;
+constexpr uint32_t kClEnterFrontier = 3840;   // and come back below these (what one CTA's queue could hold,
+constexpr unsigned long long kClEnterEdges = 16384;  // fat entries in pieces)
+constexpr uint32_t kClPiece = 64;             // edges of a piece
 
 // Single-CTA phase: when a push level's frontier fits one pass of one CTA
 // (<= blockDim.x vertices and <= 4 blockDim.x out-edges) the heuristic and
@@ -579,7 +580,12 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
         for (uint32_t k = 0; k < kmax; ++k) push_edge(u, b + k, k < mine);
       }
     } else {
-      // pull: every unvisited vertex looks for a neighbour at level L - 1
+      // pull: every unvisited vertex looks for a neighbour at level L - 1, four
+      // edges per lane in flight; vertices of more than kWarpDegree edges look
+      // at their first four (in R-MAT rows the hubs) before the warp walks the
+      // rest together.  Levels are read through L1: a line cached before a
+      // vertex got level L still says INF, and neither is L - 1 (what was
+      // written before the level's barrier is not stale after it).
       const uint32_t lane = lane_id();
       const uint32_t gw = tid >> 5, nw = nthreads >> 5;
       for (uint32_t base = gw * 32u; base < g.n; base += nw * 32u) {
@@ -587,31 +593,59 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
         bool unv = false;
         uint32_t b = 0, e = 0;
         if (v < g.n && __ldcg(a.level + v) == kInf) {
-          unv = true;
           b = __ldg(g.row + v);
           e = __ldg(g.row + v + 1);
+          unv = b < e;
         }
         const uint32_t deg = e - b;
         bool found = false;
-        if (unv && deg <= kWarpDegree) {
-          for (uint32_t j = b; j < e; ++j)
-            if (__ldcg(a.level + __ldg(g.dst + j)) == Li - 1) { found = true; break; }
+        const uint32_t lim = deg <= kWarpDegree ? e : b + 4u;
+        bool more = unv;
+        for (uint32_t k = b; __any_sync(0xffffffffu, more); k += 4) {
+          uint32_t u[4];
+          int32_t l[4];
+#pragma unroll
+          for (int r = 0; r < 4; ++r) u[r] = more && k + r < lim ? __ldg(g.dst + k + r) : kHole;
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            l[r] = kInf;
+            if (u[r] != kHole) l[r] = __ldca(a.level + u[r]);
+          }
+          const bool hit = l[0] == Li - 1 || l[1] == Li - 1 || l[2] == Li - 1 || l[3] == Li - 1;
+          found = found || hit;
+          more = more && !hit && k + 4 < lim;
         }
-        uint32_t coop = __ballot_sync(0xffffffffu, unv && deg > kWarpDegree);
+        uint32_t coop = __ballot_sync(0xffffffffu, unv && !found && deg > kWarpDegree);
         while (coop) {
           const int s = __ffs(coop) - 1;
           coop &= coop - 1;
           const uint32_t bb = __shfl_sync(0xffffffffu, b, s), ee = __shfl_sync(0xffffffffu, e, s);
           bool hit = false;
-          for (uint32_t j0 = bb; j0 < ee && !hit; j0 += 32) {
-            const uint32_t j = j0 + lane;
-            const bool h = j < ee && __ldcg(a.level + __ldg(g.dst + j)) == Li - 1;
-            hit = __ballot_sync(0xffffffffu, h) != 0u;
+          for (uint32_t j0 = bb + 4; j0 < ee && !hit; j0 += 128) {
+            uint32_t u[4];
+            int32_t l[4];
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              const uint32_t j = j0 + 32u * r + lane;
+              u[r] = j < ee ? __ldg(g.dst + j) : kHole;
+            }
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+              l[r] = kInf;
+              if (u[r] != kHole) l[r] = __ldca(a.level + u[r]);
+            }
+            hit = __any_sync(0xffffffffu, l[0] == Li - 1 || l[1] == Li - 1 || l[2] == Li - 1 || l[3] == Li - 1);
           }
           if ((int)lane == s) found = hit;
         }
         if (found) gsrb::ptx::st_relaxed_gpu_s32(a.level + v, Li);
-        discover(found, v);
+        // the new frontier's entries: the row range is known
+        const uint32_t d = found ? deg : 0u;
+        const uint2 range = make_uint2(b, e);
+        const bool reg1[1] = {found && d <= kBigDegree};
+        push_append_reg<1>(reg1, &range, sink);
+        warp_append(found && d > kBigDegree, range, hout, &c->n_big, g.n, a.overflow);
+        m_acc += d;
       }
     }
     // edge sums and entry counts of the new frontier; in a large level one
@@ -644,6 +678,7 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
 // rest the chain of trips to L2.  Here a level is: entry (shared memory) ->
 // destinations -> claims with the candidates' row ranges -> shared-memory
 // append -> records exchanged, about 1200 cycles.
+static_assert(kClEnterFrontier + kClEnterEdges / kClPiece <= kClQueue, "entries and pieces fit one CTA's queue");
 struct BfsClShared {
   uint2 q[2][kClQueue];  // edge ranges of the frontier's vertices, by parity of the level
   ClusterLink link;
@@ -684,7 +719,7 @@ __global__ void __launch_bounds__(512) bfs_init_kernel(BfsArgs a, uint32_t* flag
     *reinterpret_cast<unsigned long long*>(a.solo + 4) = (unsigned long long)g.m - (e - b);
     *reinterpret_cast<unsigned long long*>(a.solo + 6) = e - b;
     // (the policy decides a traversal's first level: that one runs on the grid)
-    a.phase[0] = e - b > kClEnterEdges || hub || a.mode == GSRB_BFS_LEARNED ? PHASE_GRID : PHASE_CLUSTER;
+    a.phase[0] = hub || a.mode == GSRB_BFS_LEARNED ? PHASE_GRID : PHASE_CLUSTER;
   }
   if (prefetch) {
     prefetch_l2(g.row, (uint64_t)(g.n + 1) * 4, tid, nt);
@@ -818,8 +853,11 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
     const uint2* qg = reinterpret_cast<const uint2*>(a.q[p]);
     const uint32_t s0 = (uint32_t)((uint64_t)slots * rank / ncta), s1 = (uint32_t)((uint64_t)slots * (rank + 1) / ncta);
     for (uint32_t i = s0 + threadIdx.x; i < s1; i += blockDim.x) {
+      // fat entries in pieces (a source of 3644 edges on one warp took 86 us)
       const uint2 r = __ldcg(qg + i);
-      if (r.y != r.x) s.q[p][atomicAdd(&s.n[p], 1u)] = r;
+      const uint32_t pieces = (r.y - r.x + kClPiece - 1) / kClPiece;
+      uint32_t at = pieces ? atomicAdd(&s.n[p], pieces) : 0u;
+      for (uint32_t b = r.x; b < r.y; b += kClPiece) s.q[p][at++] = make_uint2(b, min(b + kClPiece, r.y));
     }
   }
   uint32_t phases = 0, fl = 0, own;
@@ -3055,9 +3093,9 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
     // A kernel whose turn it is not returns at once, so the usual order is
     // queued without a look at the device: the cluster for the whole of a thin
     // graph; cluster, grid and the thin last levels on the cluster again
-    // otherwise (no cluster first for a source of more edges than it takes, or
+    // otherwise (no cluster first for a hub as the source, or
     // when the policy decides the first level).
-    const bool cluster_first = mode != GSRB_BFS_LEARNED && G->h_row[src + 1] - G->h_row[src] <= kClEnterEdges;
+    const bool cluster_first = mode != GSRB_BFS_LEARNED && G->h_row[src + 1] - G->h_row[src] <= kBigDegree;
     if (cluster_first) st = cluster();
     for (uint32_t turn = thin && cluster_first ? 0u : 1u;; ++turn) {
       if (!st && turn) st = whole();

@@ -2741,13 +2741,11 @@ int cluster_ctas(gsrb_ctx* ctx, const void* fn, size_t smem) {
   return 0;
 }
 
-gsrb_status_t finish_stats(gsrb_graph* G, gsrb_traversal_stats_t* st, float ms) {
-  uint32_t h[32];
-  unsigned long long edges = 0;
-  GSRB_CUDA(cudaStreamSynchronize(G->ctx->stream));
-  GSRB_CUDA(cudaMemcpy(h, G->flags, sizeof(h), cudaMemcpyDeviceToHost));
-  memcpy(&edges, h + 16, sizeof(edges));
+// Statistics from a copy of the graph's 32 status words.
+gsrb_status_t stats_of(const gsrb_graph* G, const uint32_t* h, gsrb_traversal_stats_t* st, float ms) {
   if (st) {
+    unsigned long long edges = 0;
+    memcpy(&edges, h + 16, sizeof(edges));
     st->levels = h[4];
     st->aux = h[5];
     st->decisions = h[6];
@@ -2760,6 +2758,22 @@ gsrb_status_t finish_stats(gsrb_graph* G, gsrb_traversal_stats_t* st, float ms) 
   if (h[0]) return GSRB_ERR_OVERFLOW;
   if (h[7]) return GSRB_ERR_TIMEOUT;
   return GSRB_OK;
+}
+
+// Enqueues the copy of the status words into the context's pinned block (slot
+// k of kSlots, 32 words each); valid after the stream has been waited for.
+cudaError_t copy_status(gsrb_graph* G, int k) {
+  return cudaMemcpyAsync(G->ctx->h_status + 32 * k, G->flags, 128, cudaMemcpyDeviceToHost, G->ctx->stream);
+}
+
+// End of a traversal (events 62 and 63 around it): one wait for the stream.
+gsrb_status_t finish_stats(gsrb_graph* G, gsrb_traversal_stats_t* st) {
+  gsrb_ctx* ctx = G->ctx;
+  GSRB_CUDA(copy_status(G, 0));
+  GSRB_CUDA(cudaStreamSynchronize(ctx->stream));
+  float ms = 0;
+  GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
+  return stats_of(G, ctx->h_status, st, ms);
 }
 
 }  // namespace
@@ -3102,18 +3116,21 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
       if (!st && turn) st = cluster();
       if (st) return st;
       GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-      uint32_t phase = 0;
-      GSRB_CUDA(cudaMemcpyAsync(&phase, a.phase, sizeof(phase), cudaMemcpyDeviceToHost, ctx->stream));
+      GSRB_CUDA(copy_status(G, 0));
       GSRB_CUDA(cudaStreamSynchronize(ctx->stream));
+      const uint32_t phase = ctx->h_status[a.phase - G->flags];
       if (phase == PHASE_DONE) break;
       // (every turn runs at least one level; n levels are the most there are)
       if ((phase != PHASE_GRID && phase != PHASE_CLUSTER) || turn > G->n) return GSRB_ERR_STATE;
     }
   }
-  GSRB_CUDA(cudaEventSynchronize(ctx->events[63]));
-  float ms = 0;
-  GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
-  st = finish_stats(G, stats, ms);
+  if (a.staged) {  // the status is here
+    float ms = 0;
+    GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
+    st = stats_of(G, ctx->h_status, stats, ms);
+  } else {
+    st = finish_stats(G, stats);
+  }
   if (stats) stats->launch = launch;
   return st;
 }
@@ -3189,10 +3206,7 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
   st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-  GSRB_CUDA(cudaEventSynchronize(ctx->events[63]));
-  float ms = 0;
-  GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
-  st = finish_stats(G, stats, ms);
+  st = finish_stats(G, stats);
   if (stats) stats->launch = launch;
   return st;
 }
@@ -3227,10 +3241,7 @@ gsrb_status_t gsrb_pagerank(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha, int32_t
   gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-  GSRB_CUDA(cudaEventSynchronize(ctx->events[63]));
-  float ms = 0;
-  GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
-  return finish_stats(G, stats, ms);
+  return finish_stats(G, stats);
 }
 
 gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha, float epsilon, int32_t max_iters,
@@ -3273,10 +3284,7 @@ gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha
   gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-  GSRB_CUDA(cudaEventSynchronize(ctx->events[63]));
-  float ms = 0;
-  GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
-  return finish_stats(G, stats, ms);
+  return finish_stats(G, stats);
 }
 
 }  // extern "C"
@@ -3515,10 +3523,12 @@ gsrb_status_t gsrb_batch_sssp(gsrb_batch_t B, const uint32_t* srcs, int32_t* con
 
 gsrb_status_t gsrb_batch_stats(gsrb_batch_t B, gsrb_traversal_stats_t* stats) {
   if (!B) return GSRB_ERR_ARG;
+  std::lock_guard<std::mutex> g(B->ctx->mu);
+  for (size_t i = 0; i < B->graphs.size(); ++i) GSRB_CUDA(copy_status(B->graphs[i], (int)i));
   GSRB_CUDA(cudaStreamSynchronize(B->ctx->stream));
   gsrb_status_t worst = GSRB_OK;
   for (size_t i = 0; i < B->graphs.size(); ++i) {
-    gsrb_status_t st = finish_stats(B->graphs[i], stats ? &stats[i] : nullptr, 0.f);
+    gsrb_status_t st = stats_of(B->graphs[i], B->ctx->h_status + 32 * i, stats ? &stats[i] : nullptr, 0.f);
     if (st && !worst) worst = st;
   }
   return worst;

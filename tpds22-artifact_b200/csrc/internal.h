@@ -27,6 +27,7 @@ struct gsrb_ctx {
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   void* stream_words = nullptr;  // scan: state line and tagged tile sums (see scan_stream_kernel)
+  uint32_t* h_status = nullptr;  // pinned: traversals' status words (kSlots x 32)
   // L2 flush buffer
   void* flush = nullptr;
   size_t flush_bytes = 0;

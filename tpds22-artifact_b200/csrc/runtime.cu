@@ -353,6 +353,7 @@ gsrb_status_t gsrb_ctx_create(int device, gsrb_ctx_t* out) {
   if (e == cudaSuccess) e = cudaMemset(c->stream_words, 0, wbytes);
   const uint32_t first_tag = 1;  // zeroed words match no round
   if (e == cudaSuccess) e = cudaMemcpy(c->stream_words, &first_tag, sizeof(first_tag), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMallocHost(&c->h_status, sizeof(uint32_t) * 32 * kSlots);
   if (e == cudaSuccess) e = cudaMemset(c->slots, 0, sbytes);
   if (e == cudaSuccess) e = cudaMemset(c->groups, 0, gbytes);
   if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -376,6 +377,7 @@ gsrb_status_t gsrb_ctx_destroy(gsrb_ctx_t c) {
   if (c->lf) cudaFree(c->lf);
   if (c->scratch) cudaFree(c->scratch);
   if (c->stream_words) cudaFree(c->stream_words);
+  if (c->h_status) cudaFreeHost(c->h_status);
   if (c->flush) cudaFree(c->flush);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);
   delete c;

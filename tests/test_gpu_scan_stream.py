@@ -98,3 +98,22 @@ def test_reduce_in_order(gsrb, ctx, n, grid):
         want.append(int(cur.astype(np.uint32).view(np.int32).astype(np.int64).sum()))
     ctx.check_status("chain")
     assert sums.download().tolist() == want
+
+
+def test_chained_reductions_behind_a_scan(gsrb, ctx):
+    """scan -> chained reduce of another array -> chained reduce of the scan's
+    output: neither reduction's predecessor writes its input, so both may be
+    chained, and the second must still see the whole scan."""
+    n = 1 << 24
+    a = np.ones(n, np.uint32)
+    d, x = ctx.to_device(a), ctx.array(n, np.uint32)
+    small = ctx.to_device(np.arange(1000, dtype=np.int32))
+    sums = ctx.array(2, np.int64).zero()
+    c = gsrb.cfg(variant=gsrb.BAR_FANOUT, ctas_per_sm=2, threads=256, overlap=1, tile=1)
+    for k in range(4):
+        x.zero()
+        gsrb.check(ctx.scan(d, x, n), "scan")
+        gsrb.check(ctx.reduce_i32(small, 1000, sums.at(0), c), "reduce")
+        gsrb.check(ctx.reduce_i32(x, n, sums.at(1), c), "reduce")
+        ctx.check_status("chain")
+        assert sums.download().tolist() == [499500, n * (n - 1) // 2]

@@ -2,8 +2,9 @@
 // worklist, pull, topology push; direction chosen per level by a fixed
 // heuristic or by the learned policy), SSSP (near-far buckets with atomicMin)
 // and pull PageRank (FP32 state, FP64 per-vertex accumulation, fixed
-// iteration count).  One kernel launch per traversal; one grid barrier per
-// level / bucket step / iteration.
+// iteration count).  One grid kernel per traversal, one grid barrier per level /
+// bucket step / iteration; thin BFS levels and thin graphs' SSSP rounds run on
+// one cluster instead (bfs_cluster_kernel, sssp_cluster_kernel).
 //
 // Reference: the GGC "outlined iterate" kernels gg_main_pipe_1_gpu_gb of
 // LONESTAR/apps/bfs/kernel_gsrb.cu:591-626 (BFS), apps/sssp/kernel_gsrb.cu:637-687
@@ -3538,6 +3539,7 @@ gsrb_status_t gsrb_batch_stats(gsrb_batch_t B, gsrb_traversal_stats_t* stats) {
 gsrb_status_t gsrb_capture_begin(gsrb_ctx_t ctx) {
   if (!ctx) return GSRB_ERR_ARG;
   GSRB_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+  ctx->writer_open = true;  // recorded and live calls do not follow one another
   return GSRB_OK;
 }
 
@@ -3545,6 +3547,7 @@ gsrb_status_t gsrb_capture_end(gsrb_ctx_t ctx, gsrb_exec_t* out) {
   if (!ctx || !out) return GSRB_ERR_ARG;
   cudaGraph_t graph = nullptr;
   GSRB_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
+  ctx->writer_open = true;
   cudaGraphExec_t exec = nullptr;
   cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);

@@ -27,6 +27,10 @@ struct gsrb_ctx {
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   void* stream_words = nullptr;  // scan: state line and tagged tile sums (see scan_stream_kernel)
+  // A kernel that writes arrays (scan, segmented scan) may still be running when
+  // the launch after it is let in early; see early_launch.  Cleared by a reduce
+  // that waits for it before it lets the next kernel in.
+  bool writer_open = false;
   uint32_t* h_status = nullptr;  // pinned: traversals' status words (kSlots x 32)
   // L2 flush buffer
   void* flush = nullptr;
@@ -82,6 +86,11 @@ gsrb::GridBarrier make_barrier(gsrb_ctx* ctx, const gsrb_cfg_t& c, int slot, uin
 // anything that kernel uses).
 gsrb_status_t launch_persistent(gsrb_ctx* ctx, const void* fn, int grid, int block, size_t smem,
                                 int cluster, int coop, void** args, bool pdl = false);
+// Whether a plain launch is made early (programmatic serialisation, waiting for
+// the kernel before it ahead of its first access, then letting the next one in):
+// on the context's own stream, which nobody else launches on, so that the
+// context knows what a chained reduction would overlap.
+inline bool early_launch(const gsrb_ctx* ctx, int coop) { return coop == 0 && ctx->stream == ctx->own_stream; }
 inline int coop_of(const gsrb_cfg_t& c) {
   if (c.variant == gsrb::V_CCG) return 2;
   return c.launch_mode == 1 ? 0 : 1;

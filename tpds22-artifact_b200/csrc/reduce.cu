@@ -107,14 +107,16 @@ reduce_i32_kernel(gsrb::GridBarrier gb, const int32_t* __restrict__ in, uint64_t
     gsrb::ptx::mbar_arrive_expect_tx(&full[buf], bytes_of(k));
     gsrb::ptx::bulk_g2s(stage + (size_t)buf * kStageBytes, src + (size_t)k * kStageBytes, bytes_of(k), &full[buf]);
   };
-  // Chained launches (pdl): the next reduction on the stream may be scheduled
-  // as soon as every CTA of this one runs; its CTAs take the SM slots this
-  // grid's CTAs free when they leave, so its stream overlaps this grid's
-  // barrier and combine.  It reads only its own input before griddep_wait.
-  // In order (kInOrder, what a plain call gets: 2^24 at 2 x 256, 16.6 -> 14.9 us
+  // Chained launches: the next reduction on the stream may be scheduled as soon
+  // as every CTA of this one runs; its CTAs take the SM slots this grid's CTAs
+  // free when they leave, so its stream overlaps this grid's barrier and combine
+  // (let in after this one's wait instead, 15.2 us a reduction for 9.6).  It reads only its own input before griddep_wait.
+  // In order (kInOrder, what a plain call gets: 2^24 at 2 x 256, 16.6 -> 15.0 us
   // back to back) a CTA waits for the kernel before
   // it ahead of its first access: only its launch and set-up overlap.
-  if (pdl) gsrb::ptx::griddep_launch_dependents();
+  // The kernel after it is let in only then: a chained one reads its input at
+  // once and counts on the kernel right before it alone not writing that.
+  if (pdl == kChained) gsrb::ptx::griddep_launch_dependents();
   // The first copies go out before the barrier's set-up reads (two dependent
   // L2 round trips): they only read the input.  Whatever the set-up decides,
   // every issued copy is waited for below before the CTA leaves.
@@ -126,7 +128,10 @@ reduce_i32_kernel(gsrb::GridBarrier gb, const int32_t* __restrict__ in, uint64_t
     }
     gsrb::ptx::fence_mbar_init();
   }
-  if (pdl == kInOrder) gsrb::ptx::griddep_wait();
+  if (pdl == kInOrder) {
+    gsrb::ptx::griddep_wait();
+    gsrb::ptx::griddep_launch_dependents();
+  }
   if (tid < head) acc += ph[tid];
   if (tid < tail) acc += p[(nbytes >> 2) + tid];
   if (tid == 0) {
@@ -263,9 +268,15 @@ extern "C" gsrb_status_t gsrb_reduce_i32(gsrb_ctx_t ctx, const int32_t* d_in, si
   const size_t smem = gsrb_reduce_smem_for(c);
   uint32_t nbuf = (uint32_t)(smem / kStageBytes);
   // chained launch: plain launches only (a cooperative launch is refused)
-  const bool pdl = coop_of(c) == 0;
-  if (c.overlap != 0 && !pdl) return GSRB_ERR_UNSUPPORTED;
-  uint32_t pdl32 = !pdl ? 0u : (c.overlap != 0 ? kChained : kInOrder);
+  const int coop = coop_of(c);
+  if (c.overlap != 0 && coop != 0) return GSRB_ERR_UNSUPPORTED;
+  const bool chained = c.overlap != 0;
+  uint32_t pdl32 = chained ? (uint32_t)kChained : early_launch(ctx, coop) ? (uint32_t)kInOrder : 0u;
+  // A chained launch lets the next one in at once, and that one must not meet a
+  // kernel that may be writing its input: behind such a kernel it waits in line.
+  const bool pdl = chained ? !ctx->writer_open : pdl32 == kInOrder;
   void* args[] = {&gb, &d_in, &n64, &partials, &out, &nbuf, &pdl32};
-  return launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop_of(c), args, pdl);
+  st = launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop, args, pdl);
+  if (!st) ctx->writer_open = false;
+  return st;
 }

@@ -388,6 +388,7 @@ gsrb_status_t gsrb_ctx_set_stream(gsrb_ctx_t c, void* stream) {
   if (!c) return GSRB_ERR_ARG;
   std::lock_guard<std::mutex> g(c->mu);
   c->stream = stream ? (cudaStream_t)stream : c->own_stream;
+  c->writer_open = true;  // (what ran on that stream last is not known here)
   return GSRB_OK;
 }
 

@@ -661,7 +661,7 @@ template <bool F32, int V>
 __global__ void __launch_bounds__(kStreamThreads, 1)
 scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __restrict__ in,
                    typename ScanT<F32>::Elem* __restrict__ out, uint64_t n, StreamState* st,
-                   unsigned long long* __restrict__ words) {
+                   unsigned long long* __restrict__ words, uint32_t early) {
   using Elem = typename ScanT<F32>::Elem;
   using Acc = typename ScanT<F32>::Acc;
   using Vec = typename ScanT<F32>::Vec;
@@ -700,10 +700,9 @@ scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __rest
   auto slot = [&](uint32_t round, uint32_t cta) {
     return words + ((size_t)(round % kStreamRounds) * G + cta) * NW;
   };
-  // The next kernel on the stream may be scheduled (not run past its own wait)
-  // while this one works, and this one was scheduled early the same way: the
-  // set-up below overlaps the kernel before it, nothing else does.
-  gsrb::ptx::griddep_launch_dependents();
+  // This grid may be scheduled while the kernel before it on the stream still
+  // works: the set-up below overlaps it, nothing else does.  The next one is
+  // let in the same way once that kernel has finished.
   if (tid == 0) {
     for (uint32_t k = 0; k < kStreamStages; ++k) {
       gsrb::ptx::mbar_init(&full[k], 1);
@@ -717,6 +716,7 @@ scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __rest
     s_fail = 0;
   }
   gsrb::ptx::griddep_wait();
+  if (early) gsrb::ptx::griddep_launch_dependents();
   if (tid == 0) {
     for (uint32_t i = 0; i < mine && i < kStreamStages; ++i) issue(i);
   }
@@ -934,9 +934,11 @@ gsrb_status_t stream_launch(gsrb_ctx* ctx, const void* d_in, void* d_out, uint64
   gsrb::GridBarrier gb = make_barrier(ctx, c, 0, (uint32_t)grid, 0, 0);
   StreamState* st = reinterpret_cast<StreamState*>(ctx->stream_words);
   unsigned long long* words = reinterpret_cast<unsigned long long*>(st + 1);
-  void* args[] = {&gb, (void*)&d_in, &d_out, &n, &st, &words};
+  uint32_t early = early_launch(ctx, 0) ? 1u : 0u;
+  if (early) ctx->writer_open = true;
+  void* args[] = {&gb, (void*)&d_in, &d_out, &n, &st, &words, &early};
   return launch_persistent(ctx, fn, grid, (int)kStreamThreads, (size_t)kStreamStages * tile * 4u, 1, 0, args,
-                           true);
+                           early != 0);
 }
 
 gsrb_status_t scan_launch(gsrb_ctx_t ctx, const void* d_in, void* d_out, size_t n, const gsrb_cfg_t* cfgin,

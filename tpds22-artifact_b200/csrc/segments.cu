@@ -44,6 +44,7 @@ struct SegParams {
   gsrb::GridBarrier gb;   // slot 1's descriptor (nparticipants/first_cta set per segment)
   uint64_t flip_stride;   // words between consecutive slots' flip areas
   uint32_t k;
+  uint32_t early;         // launched early: let the next kernel in once the one before has finished
   uint32_t chunk;         // scan: elements per CTA per round (whole tiles of kScanV x blockDim)
   uint64_t off[kMaxSegments + 1];
 };
@@ -197,10 +198,10 @@ reduce_segments_kernel(SegParams p, const int32_t* __restrict__ in, long long* _
   __shared__ gsrb::BarrierShared bsh;
   __shared__ long long buf[32];
   __shared__ uint32_t s_comb;
-  gsrb::ptx::griddep_launch_dependents();  // see launch_segments
   const SegTeam t = seg_team(p);
   gsrb::GridSync<V> bar;
-  gsrb::ptx::griddep_wait();
+  gsrb::ptx::griddep_wait();  // see launch_segments
+  if (p.early) gsrb::ptx::griddep_launch_dependents();
   const bool ok = bar.init(seg_barrier(p, t), &bsh);
   long long s = 0;
   if (ok) s = slice_sum_i32(in, t.a, t.b);
@@ -300,10 +301,10 @@ scan_segments_kernel(SegParams p, const T* __restrict__ in, T* __restrict__ out,
   __shared__ T wsum[32];
   extern __shared__ __align__(16) unsigned char tile_raw[];  // tpos(kScanV * blockDim) elements
   T* tile = reinterpret_cast<T*>(tile_raw);
-  gsrb::ptx::griddep_launch_dependents();  // see launch_segments
   const SegTeam t = seg_team(p);
   gsrb::GridSync<V> bar;
-  gsrb::ptx::griddep_wait();
+  gsrb::ptx::griddep_wait();  // see launch_segments
+  if (p.early) gsrb::ptx::griddep_launch_dependents();
   bool ok = bar.init(seg_barrier(p, t), &bsh);
   const uint64_t o0 = p.off[t.seg], o1 = p.off[t.seg + 1];
   const uint64_t C = p.chunk, R = C * t.count;
@@ -466,11 +467,11 @@ scan_segments_reg_kernel(SegParams p, const T* __restrict__ in, T* __restrict__ 
   const bool leader = gt == 0;
   const uint32_t NB = NG + 2;
   const uint64_t C = (uint64_t)GT * D * 4u;  // elements of one CTA's chunk
-  gsrb::ptx::griddep_launch_dependents();  // see launch_segments
   const SegTeam t = seg_team(p);
   const gsrb::GridBarrier gb = seg_barrier(p, t);
   gsrb::GridSync<gsrb::V_FANOUT> bar;
-  gsrb::ptx::griddep_wait();
+  gsrb::ptx::griddep_wait();  // see launch_segments
+  if (p.early) gsrb::ptx::griddep_launch_dependents();
   const bool ok0 = bar.init(gb, &bsh);
   if (tid == 0) {
     s_epoch0 = bar.epoch;
@@ -635,8 +636,11 @@ const void* scan_segments_fn(int v) {
 // Plain launches are made early (programmatic serialisation): the layout search
 // over the offsets overlaps the kernel before this one on the stream, which is
 // waited for ahead of the first access.
-gsrb_status_t launch_segments(gsrb_ctx* ctx, const void* fn, int grid, const gsrb_cfg_t& c, size_t smem, void** args) {
-  return launch_persistent(ctx, fn, grid, c.threads, smem, 1, coop_of(c), args, coop_of(c) == 0);
+gsrb_status_t launch_segments(gsrb_ctx* ctx, const void* fn, int grid, const gsrb_cfg_t& c, size_t smem, SegParams* p,
+                              void** args) {
+  p->early = early_launch(ctx, coop_of(c)) ? 1u : 0u;
+  if (p->early) ctx->writer_open = true;
+  return launch_persistent(ctx, fn, grid, c.threads, smem, 1, coop_of(c), args, p->early != 0);
 }
 
 // Shared checks and the launch parameters of a segmented call.
@@ -707,7 +711,7 @@ gsrb_status_t scan_segments(gsrb_ctx* ctx, const T* d_in, T* d_out, const uint64
     Acc* partials = (Acc*)part;
     const void* rf = scan_segments_reg_fn<T>(wide);
     void* args[] = {&p, &d_in, &d_out, &partials, &ng};
-    return launch_segments(ctx, rf, grid, c, 0, args);
+    return launch_segments(ctx, rf, grid, c, 0, &p, args);
   }
   st = scratch(ctx, sizeof(Acc) * 2 * (size_t)grid, &part);
   if (st) return st;
@@ -715,7 +719,7 @@ gsrb_status_t scan_segments(gsrb_ctx* ctx, const T* d_in, T* d_out, const uint64
   const uint32_t tw = kScanV * (uint32_t)c.threads;
   const size_t smem = sizeof(T) * (size_t)(tw + (tw >> 5));
   void* args[] = {&p, &d_in, &d_out, &partials};
-  return launch_segments(ctx, fn, grid, c, smem, args);
+  return launch_segments(ctx, fn, grid, c, smem, &p, args);
 }
 
 }  // namespace
@@ -750,7 +754,7 @@ gsrb_status_t gsrb_reduce_i32_segments(gsrb_ctx_t ctx, const int32_t* d_in, cons
   long long* partials = (long long*)part;
   long long* out = (long long*)d_out;
   void* args[] = {&p, &d_in, &partials, &out};
-  return launch_segments(ctx, fn, grid, c, 0, args);
+  return launch_segments(ctx, fn, grid, c, 0, &p, args);
 }
 
 gsrb_status_t gsrb_scan_u32_segments(gsrb_ctx_t ctx, const uint32_t* d_in, uint32_t* d_out, const uint64_t* h_off,

@@ -2761,16 +2761,17 @@ gsrb_status_t stats_of(const gsrb_graph* G, const uint32_t* h, gsrb_traversal_st
   return GSRB_OK;
 }
 
-// Enqueues the copy of the status words into the context's pinned block (slot
-// k of kSlots, 32 words each); valid after the stream has been waited for.
-cudaError_t copy_status(gsrb_graph* G, int k) {
-  return cudaMemcpyAsync(G->ctx->h_status + 32 * k, G->flags, 128, cudaMemcpyDeviceToHost, G->ctx->stream);
+// Enqueues the copy of the status words into the pinned block (slot k of kSlots,
+// 32 words each) of the context that runs the traversal, on its stream; valid
+// after that stream has been waited for.  (A graph may be used from another
+// context than the one it was made on.)
+cudaError_t copy_status(gsrb_ctx* ctx, const gsrb_graph* G, int k) {
+  return cudaMemcpyAsync(ctx->h_status + 32 * k, G->flags, 128, cudaMemcpyDeviceToHost, ctx->stream);
 }
 
-// End of a traversal (events 62 and 63 around it): one wait for the stream.
-gsrb_status_t finish_stats(gsrb_graph* G, gsrb_traversal_stats_t* st) {
-  gsrb_ctx* ctx = G->ctx;
-  GSRB_CUDA(copy_status(G, 0));
+// End of a traversal (the context's events 62 and 63 around it): one wait for the stream.
+gsrb_status_t finish_stats(gsrb_ctx* ctx, const gsrb_graph* G, gsrb_traversal_stats_t* st) {
+  GSRB_CUDA(copy_status(ctx, G, 0));
   GSRB_CUDA(cudaStreamSynchronize(ctx->stream));
   float ms = 0;
   GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
@@ -3117,7 +3118,7 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
       if (!st && turn) st = cluster();
       if (st) return st;
       GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-      GSRB_CUDA(copy_status(G, 0));
+      GSRB_CUDA(copy_status(ctx, G, 0));
       GSRB_CUDA(cudaStreamSynchronize(ctx->stream));
       const uint32_t phase = ctx->h_status[a.phase - G->flags];
       if (phase == PHASE_DONE) break;
@@ -3130,7 +3131,7 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
     GSRB_CUDA(cudaEventElapsedTime(&ms, ctx->events[62], ctx->events[63]));
     st = stats_of(G, ctx->h_status, stats, ms);
   } else {
-    st = finish_stats(G, stats);
+    st = finish_stats(ctx, G, stats);
   }
   if (stats) stats->launch = launch;
   return st;
@@ -3207,7 +3208,7 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
   st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-  st = finish_stats(G, stats);
+  st = finish_stats(ctx, G, stats);
   if (stats) stats->launch = launch;
   return st;
 }
@@ -3242,7 +3243,7 @@ gsrb_status_t gsrb_pagerank(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha, int32_t
   gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-  return finish_stats(G, stats);
+  return finish_stats(ctx, G, stats);
 }
 
 gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha, float epsilon, int32_t max_iters,
@@ -3285,7 +3286,7 @@ gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha
   gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
-  return finish_stats(G, stats);
+  return finish_stats(ctx, G, stats);
 }
 
 }  // extern "C"
@@ -3525,7 +3526,7 @@ gsrb_status_t gsrb_batch_sssp(gsrb_batch_t B, const uint32_t* srcs, int32_t* con
 gsrb_status_t gsrb_batch_stats(gsrb_batch_t B, gsrb_traversal_stats_t* stats) {
   if (!B) return GSRB_ERR_ARG;
   std::lock_guard<std::mutex> g(B->ctx->mu);
-  for (size_t i = 0; i < B->graphs.size(); ++i) GSRB_CUDA(copy_status(B->graphs[i], (int)i));
+  for (size_t i = 0; i < B->graphs.size(); ++i) GSRB_CUDA(copy_status(B->ctx, B->graphs[i], (int)i));
   GSRB_CUDA(cudaStreamSynchronize(B->ctx->stream));
   gsrb_status_t worst = GSRB_OK;
   for (size_t i = 0; i < B->graphs.size(); ++i) {

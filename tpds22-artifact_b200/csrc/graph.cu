@@ -3539,6 +3539,7 @@ gsrb_status_t gsrb_batch_stats(gsrb_batch_t B, gsrb_traversal_stats_t* stats) {
 // ---- CUDA graphs: capture the context stream's work once, replay it ----------
 gsrb_status_t gsrb_capture_begin(gsrb_ctx_t ctx) {
   if (!ctx) return GSRB_ERR_ARG;
+  std::lock_guard<std::mutex> g(ctx->mu);
   GSRB_CUDA(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
   ctx->writer_open = true;  // recorded and live calls do not follow one another
   return GSRB_OK;
@@ -3547,8 +3548,11 @@ gsrb_status_t gsrb_capture_begin(gsrb_ctx_t ctx) {
 gsrb_status_t gsrb_capture_end(gsrb_ctx_t ctx, gsrb_exec_t* out) {
   if (!ctx || !out) return GSRB_ERR_ARG;
   cudaGraph_t graph = nullptr;
-  GSRB_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
-  ctx->writer_open = true;
+  {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    GSRB_CUDA(cudaStreamEndCapture(ctx->stream, &graph));
+    ctx->writer_open = true;
+  }
   cudaGraphExec_t exec = nullptr;
   cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
   cudaGraphDestroy(graph);
@@ -3559,7 +3563,9 @@ gsrb_status_t gsrb_capture_end(gsrb_ctx_t ctx, gsrb_exec_t* out) {
 
 gsrb_status_t gsrb_exec_launch(gsrb_ctx_t ctx, gsrb_exec_t exec) {
   if (!ctx || !exec) return GSRB_ERR_ARG;
+  std::lock_guard<std::mutex> g(ctx->mu);
   GSRB_CUDA(cudaGraphLaunch((cudaGraphExec_t)exec, ctx->stream));
+  ctx->writer_open = true;  // (the replay may end in a kernel that lets the next one in)
   g_launches.fetch_add(1, std::memory_order_relaxed);
   return GSRB_OK;
 }

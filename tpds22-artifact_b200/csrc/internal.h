@@ -27,9 +27,9 @@ struct gsrb_ctx {
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
   void* stream_words = nullptr;  // scan: state line and tagged tile sums (see scan_stream_kernel)
-  // A kernel that writes arrays (scan, segmented scan) may still be running when
-  // the launch after it is let in early; see early_launch.  Cleared by a reduce
-  // that waits for it before it lets the next kernel in.
+  // A kernel that writes arrays (scan, segmented scan, a reduce's result) may
+  // still be running when the launch after it is let in early; see early_launch.
+  // Cleared by a launch that waits for it in line and lets nobody in before.
   bool writer_open = false;
   uint32_t* h_status = nullptr;  // pinned: traversals' status words (kSlots x 32)
   // L2 flush buffer

@@ -277,6 +277,7 @@ extern "C" gsrb_status_t gsrb_reduce_i32(gsrb_ctx_t ctx, const int32_t* d_in, si
   const bool pdl = chained ? !ctx->writer_open : pdl32 == kInOrder;
   void* args[] = {&gb, &d_in, &n64, &partials, &out, &nbuf, &pdl32};
   st = launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop, args, pdl);
-  if (!st) ctx->writer_open = false;
+  // In order, this launch lets the next one in while it still has to write *d_out.
+  if (!st) ctx->writer_open = pdl32 == kInOrder;
   return st;
 }

@@ -58,3 +58,23 @@ def test_behind_a_replay(gsrb, ctx, arrays):
         ctx.check_status("chain")
         assert d["res"].download().tolist() == [d["want"], 499500, d["want"], 0]
     g.free()
+
+
+def test_behind_chained_reductions(gsrb, ctx, arrays):
+    """Every third call reads the result of the chained call before the one
+    before it; more results than the context keeps in mind."""
+    d, chained = arrays, _cfg(gsrb, overlap=1)
+    k = 100
+    res = ctx.array(3 * k, np.int64).zero()
+    for i in range(k):
+        gsrb.check(ctx.reduce_i32(d["big"], N, res.at(3 * i), chained), "chained")
+        gsrb.check(ctx.reduce_i32(d["small"], 1000, res.at(3 * i + 1), chained), "chained")
+        gsrb.check(ctx.reduce_i32(res.at(3 * i), 2, res.at(3 * i + 2), chained), "chained")
+    ctx.check_status("chain")
+    assert res.download().tolist() == [d["want"], 499500, d["want"]] * k
+    res.zero()
+    for i in range(k):  # as many results without a reader: the chain starts over when the list is full
+        gsrb.check(ctx.reduce_i32(d["small"], 1000, res.at(i), chained), "chained")
+    gsrb.check(ctx.reduce_i32(res, 2 * k, res.at(k), chained), "chained")
+    ctx.check_status("chain")
+    assert res.download().tolist()[:k + 1] == [499500] * k + [499500 * k]

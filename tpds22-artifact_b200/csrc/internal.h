@@ -31,6 +31,12 @@ struct gsrb_ctx {
   // still be running when the launch after it is let in early; see early_launch.
   // Cleared by a launch that waits for it in line and lets nobody in before.
   bool writer_open = false;
+  // Results of the chained reductions since the last launch made in line: a
+  // chained launch starts when the one before it does, so any of them may still
+  // be missing.
+  static constexpr int kOpenResults = 64;
+  const void* open_results[kOpenResults] = {};
+  int open_n = 0;
   uint32_t* h_status = nullptr;  // pinned: traversals' status words (kSlots x 32)
   // L2 flush buffer
   void* flush = nullptr;

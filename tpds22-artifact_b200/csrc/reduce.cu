@@ -20,6 +20,8 @@
 // against a serial int64 sum.
 #include "internal.h"
 
+#include <algorithm>
+
 using namespace gsrbrt;
 
 namespace {
@@ -238,6 +240,20 @@ size_t gsrb_reduce_smem_for(const gsrb_cfg_t& c) {
   return (size_t)nb * kStageBytes;
 }
 
+namespace {
+// Whether n int32 at d_in may hold a result that a chained reduction has yet to
+// write (or there are too many of those to tell).
+bool reads_open_result(const gsrb_ctx* ctx, const int32_t* d_in, size_t n) {
+  if (ctx->open_n == gsrb_ctx::kOpenResults) return true;
+  const uintptr_t a = (uintptr_t)d_in, b = a + n * sizeof(int32_t);
+  for (int i = 0; i < ctx->open_n; ++i) {
+    const uintptr_t r = (uintptr_t)ctx->open_results[i];
+    if (r < b && a < r + sizeof(int64_t)) return true;
+  }
+  return false;
+}
+}  // namespace
+
 extern "C" gsrb_status_t gsrb_reduce_i32(gsrb_ctx_t ctx, const int32_t* d_in, size_t n, int64_t* d_out,
                                          const gsrb_cfg_t* cfgin) {
   if (!ctx || !d_out || (n && !d_in)) return GSRB_ERR_ARG;
@@ -273,11 +289,18 @@ extern "C" gsrb_status_t gsrb_reduce_i32(gsrb_ctx_t ctx, const int32_t* d_in, si
   const bool chained = c.overlap != 0;
   uint32_t pdl32 = chained ? (uint32_t)kChained : early_launch(ctx, coop) ? (uint32_t)kInOrder : 0u;
   // A chained launch lets the next one in at once, and that one must not meet a
-  // kernel that may be writing its input: behind such a kernel it waits in line.
-  const bool pdl = chained ? !ctx->writer_open : pdl32 == kInOrder;
+  // kernel that may be writing its input: behind such a kernel, or where its
+  // input holds the result of a chained reduction before it, it waits in line.
+  const bool pdl = chained ? !ctx->writer_open && !reads_open_result(ctx, d_in, n) : pdl32 == kInOrder;
   void* args[] = {&gb, &d_in, &n64, &partials, &out, &nbuf, &pdl32};
   st = launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop, args, pdl);
   // In order, this launch lets the next one in while it still has to write *d_out.
   if (!st) ctx->writer_open = pdl32 == kInOrder;
+  if (!st && !(chained && pdl)) ctx->open_n = 0;
+  if (!st && chained) {
+    const void* const* end = ctx->open_results + ctx->open_n;
+    if (std::find<const void* const*, const void*>(ctx->open_results, end, d_out) == end)
+      ctx->open_results[ctx->open_n++] = d_out;
+  }
   return st;
 }

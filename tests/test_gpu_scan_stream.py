@@ -117,3 +117,22 @@ def test_chained_reductions_behind_a_scan(gsrb, ctx):
         gsrb.check(ctx.reduce_i32(x, n, sums.at(1), c), "reduce")
         ctx.check_status("chain")
         assert sums.download().tolist() == [499500, n * (n - 1) // 2]
+
+
+@pytest.mark.parametrize("big", [1e30, np.inf])
+@pytest.mark.parametrize("n", [2048, 5000, 148 * 8192 * 2 + 77])
+def test_scan_f32_wide_range(gsrb, ctx, n, big):
+    """A value that swallows (or makes infinite) every sum behind it leaves the
+    prefixes before it as they are."""
+    for at in (0, n // 2, n // 2 + 77, n - 2):
+        a = np.ones(n, np.float32)
+        a[at] = big
+        d, o = ctx.to_device(a), ctx.array(n, np.float32)
+        gsrb.check(ctx.scan(d, o, n), "scan")
+        ctx.check_status("scan")
+        ref = np.concatenate([[0.0], np.cumsum(a[:-1].astype(np.float64))])
+        got = o.download()
+        assert np.all(np.isinf(got) == np.isinf(ref)) and not np.any(np.isnan(got))
+        fin = np.isfinite(ref)
+        # FP32 within a warp's 128 elements (seven roundings), FP64 between, one rounding of the result
+        assert np.all(np.abs(got[fin] - ref[fin]) <= 8 * 2.0**-24 * ref[fin])

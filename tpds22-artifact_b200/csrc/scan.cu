@@ -70,6 +70,16 @@ __device__ __forceinline__ void acc_from(uint64_t b, double& a) { a = __longlong
 __device__ __forceinline__ uint32_t shfl_up_acc(uint32_t v, int o) { return __shfl_up_sync(0xffffffffu, v, o); }
 __device__ __forceinline__ double shfl_up_acc(double v, int o) { return __shfl_up_sync(0xffffffffu, v, o); }
 
+// A lane's exclusive prefix from the inclusive ones.  Integers subtract; floating
+// values come from the lane before, since behind a value that is infinite or
+// much larger than what precedes it the difference is not the prefix.
+__device__ __forceinline__ uint32_t exclusive_of(uint32_t incl, uint32_t own) { return incl - own; }
+template <typename T>
+__device__ __forceinline__ T exclusive_of(T incl, T) {
+  const T y = __shfl_up_sync(0xffffffffu, incl, 1);
+  return (threadIdx.x & 31u) == 0u ? T(0) : y;
+}
+
 template <typename Acc>
 __device__ __forceinline__ Acc warp_sum(Acc v) {
 #pragma unroll
@@ -744,7 +754,7 @@ scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __rest
           const Elem y = shfl_up(incl, o);
           if ((int)lane >= o) incl += y;
         }
-        le[r] = incl - lt;
+        le[r] = exclusive_of(incl, lt);
         rt[r] = shfl_idx(incl, 31);
       }
       if (!stream_wait(&offs[q8], ph8, gb) || !stream_wait(&pref[q8], ph8, gb)) break;
@@ -799,7 +809,8 @@ scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __rest
           const Acc y = shfl_up_acc(inc, o);
           if ((int)lane >= o) inc += y;
         }
-        if (lane < kStreamWarps) s_off[q8][lane] = inc - v;
+        const Acc exc = exclusive_of(inc, v);
+        if (lane < kStreamWarps) s_off[q8][lane] = exc;
         if (lane == kStreamWarps - 1) stream_publish(slot(i, b), base + i, inc);
         __syncwarp();
         if (lane == 0) gsrb::ptx::mbar_arrive(&offs[q8]);

@@ -187,3 +187,22 @@ def test_bfs_pull_rows(gsrb, ctx, orc, path_graphs, name, mode):
             want = orc.bfs(g, src)
             assert np.array_equal(out.download(), want)
             assert st.edges == orc.traversed_edges(g, want)
+
+
+@pytest.mark.parametrize("tail", [1, 700])
+def test_sssp_vertices_without_out_edges(gsrb, ctx, orc, tail):
+    """Directed rows that end at the arrays' end: nothing is read for them."""
+    n = 1500
+    src = np.concatenate([np.arange(n - 1), np.arange(tail) % n])
+    dst = np.concatenate([np.arange(1, n), n + np.arange(tail)])
+    g = gsrb.csr_from_edges(n + tail, src, dst, symmetrize=False)
+    dg = ctx.graph(g)
+    out = ctx.array(g.nnodes, np.int32)
+    for source in (0, n + tail - 1):
+        for delta in (50, 1 << 30):
+            rc, st = dg.sssp(source, out, delta)
+            gsrb.check(rc, "sssp")
+            assert np.array_equal(out.download(), orc.dijkstra(g, source))
+        rc, st = dg.bfs(source, out)
+        gsrb.check(rc, "bfs")
+        assert np.array_equal(out.download(), orc.bfs(g, source))

@@ -1503,9 +1503,13 @@ __device__ __forceinline__ void sssp_cl_push(const SsspArgs& a, SsspClShared& s,
 #pragma unroll
   for (int r = 0; r < K; ++r) {
     const bool imp = ((act >> r) & 1u) && nd[r] < old[r], near = imp && nd[r] < T;
-    if (near) {  // the first edges are on their way to the SM while the round ends
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(g.dst + rg[r].x));
-      asm volatile("prefetch.global.L1 [%0];" ::"l"(g.w + rg[r].x));
+    if (near) {
+      // the first edges are on their way to the SM while the round ends (a row
+      // without edges may begin at the arrays' end; a test for that in place of
+      // the clamp took 2.5 % of a 2048^2 grid)
+      const uint32_t j0 = min(rg[r].x, g.m - 1u);
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(g.dst + j0));
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(g.w + j0));
     }
     sssp_cl_near(a, s, o, near, make_uint4(v[r], rg[r].x, rg[r].y, (uint32_t)nd[r]));
     sssp_cl_far(a, s, o, f, imp && !near, v[r], nd[r]);

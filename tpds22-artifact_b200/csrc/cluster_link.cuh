@@ -21,6 +21,7 @@ constexpr uint32_t kClThreads = 512;  // threads per CTA (every warp goes throug
 struct ClusterLink {
   uint4 tab[2][kClMaxCtas];  // the CTAs' records, by parity of the step
   uint64_t mbar[2];
+  uint64_t meet;             // see link_meet
 };
 
 __device__ __forceinline__ void st_async_v4(uint32_t caddr, uint4 v, uint32_t cmbar) {
@@ -37,10 +38,20 @@ __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* mbar, uint32_t p
   return ok != 0;
 }
 
+// Waits are bounded, and a wait that ran out must not leave a CTA's threads in
+// different places: a record that comes at the deadline is seen by some of them.
+// So a verdict is a warp's (link_wait, link_meet), and a CTA's warps compare
+// theirs at the barrier that ends each step and at one after the loop
+// (link_agree): a warp that gave up goes to the latter while the others go
+// through the step, and both find out there.  Nothing in between may wait for the
+// CTA or, without a bound, for the cluster.
+__device__ __forceinline__ bool link_agree(bool ok) { return __syncthreads_or(!ok) == 0; }
+
 // Thread 0 of every CTA; a cluster barrier must follow before the first use.
-__device__ __forceinline__ void link_init(ClusterLink& l) {
+__device__ __forceinline__ void link_init(ClusterLink& l, uint32_t ncta) {
   gsrb::ptx::mbar_init(&l.mbar[0], 1);
   gsrb::ptx::mbar_init(&l.mbar[1], 1);
+  gsrb::ptx::mbar_init(&l.meet, ncta);
   gsrb::ptx::fence_mbar_init();
 }
 // Thread 0, once per step before it publishes: this step's records to come.
@@ -54,21 +65,41 @@ __device__ __forceinline__ void link_publish(ClusterLink& l, uint32_t p, uint4 r
     st_async_v4(gsrb::ptx::mapa_shared(gsrb::ptx::smem_u32(&l.tab[p][rank]), lane), rec,
                 gsrb::ptx::mapa_shared(gsrb::ptx::smem_u32(&l.mbar[p]), lane));
 }
-// Every thread: all records of the step are here (bounded by timeout_ns).
+// One warp: the phase has completed before the deadline (the same in every lane).
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* mbar, uint32_t parity, uint64_t timeout_ns) {
+  uint64_t t0 = 0;
+  bool ok = false;
+  for (uint32_t it = 0; !ok; ++it) {
+    ok = mbar_try_wait_cluster(mbar, parity);
+    if ((it & 63u) == 63u) {
+      const uint64_t now = gsrb::ptx::globaltimer_ns();
+      if (t0 == 0) t0 = now;
+      else if (now - t0 > timeout_ns) break;
+    }
+  }
+  return __all_sync(0xffffffffu, ok) != 0;
+}
+// Every warp: all records of the step are here (bounded by timeout_ns).
 // Buffers alternate by the step's parity: a CTA publishes step s + 2 only after
 // every CTA published s + 1, that is after it has read the records of s.
 __device__ __forceinline__ bool link_wait(ClusterLink& l, uint32_t p, uint32_t& phases, uint64_t timeout_ns) {
   const uint32_t parity = (phases >> p) & 1u;
   phases ^= 1u << p;
-  uint64_t t0 = 0;
-  for (uint32_t it = 0;; ++it) {
-    if (mbar_try_wait_cluster(&l.mbar[p], parity)) return true;
-    if ((it & 63u) == 63u) {
-      const uint64_t now = gsrb::ptx::globaltimer_ns();
-      if (t0 == 0) t0 = now;
-      else if (now - t0 > timeout_ns) return false;
-    }
+  return mbar_wait_cluster(&l.mbar[p], parity, timeout_ns);
+}
+// Every warp: what the CTAs wrote to their shared memory before their last CTA
+// barrier can be read from all of them (bounded; the third bit of `phases` is
+// its parity).  barrier.cluster would wait without a bound, and would let a CTA
+// that gave up leave while its memory is read.
+__device__ __forceinline__ bool link_meet(ClusterLink& l, uint32_t& phases, uint32_t ncta, uint64_t timeout_ns) {
+  if (threadIdx.x < ncta) {
+    const uint32_t there = gsrb::ptx::mapa_shared(gsrb::ptx::smem_u32(&l.meet), threadIdx.x);
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(there) : "memory");
   }
+  __syncwarp();
+  const uint32_t parity = (phases >> 2) & 1u;
+  phases ^= 4u;
+  return mbar_wait_cluster(&l.meet, parity, timeout_ns);
 }
 
 __device__ __forceinline__ uint2 ld_cluster_v2(uint32_t caddr) {
@@ -83,13 +114,15 @@ __device__ __forceinline__ uint4 ld_cluster_v4(uint32_t caddr) {
   return v;
 }
 
-// A step's totals from its records, the same in every CTA (redux.sync, no shuffles).
+// A step's totals from its records, the same in every CTA (redux.sync, no
+// shuffles).  ALWAYS_Y: y counts in every step, else only beside a w.
 struct LinkSum {
   uint32_t x, y, z;  // sums of the first three fields
-  bool any;          // some CTA's y or w is set
+  bool w;            // some CTA's w is set
   uint32_t own;      // this CTA's x
   uint32_t max_x;
 };
+template <bool ALWAYS_Y>
 __device__ __forceinline__ LinkSum link_sum(const ClusterLink& l, uint32_t p, uint32_t rank, uint32_t ncta) {
   const uint32_t lane = lane_id();
   uint4 t = make_uint4(0, 0, 0, 0);
@@ -99,8 +132,8 @@ __device__ __forceinline__ LinkSum link_sum(const ClusterLink& l, uint32_t p, ui
   s.x = __reduce_add_sync(0xffffffffu, t.x);
   s.max_x = __reduce_max_sync(0xffffffffu, t.x);
   s.z = __reduce_add_sync(0xffffffffu, t.z);
-  s.any = __any_sync(0xffffffffu, (t.y | t.w) != 0u);
-  s.y = s.any ? __reduce_add_sync(0xffffffffu, t.y) : 0u;
+  s.w = __any_sync(0xffffffffu, t.w != 0u);
+  s.y = ALWAYS_Y || s.w ? __reduce_add_sync(0xffffffffu, t.y) : 0u;
   return s;
 }
 // Entries a warp takes at a time of n over the CTA's warps (at most 32).

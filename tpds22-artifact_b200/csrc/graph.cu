@@ -840,7 +840,7 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
   unsigned long long mf = __ldcg(&a.cnt[(L - 1) % 3].m_next);
   const uint32_t slots = (uint32_t)__ldcg(&a.cnt[(L - 1) % 3].n_reg);
   if (threadIdx.x == 0) {
-    link_init(s.link);
+    link_init(s.link, ncta);
     s.n[0] = s.n[1] = s.extra[0] = s.extra[1] = s.empty[0] = s.empty[1] = s.m[0] = s.m[1] = 0;
     s.fat[0] = s.fat[1] = 3u;  // of the entries read below nothing is known
   }
@@ -862,7 +862,7 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
     }
   }
   uint32_t phases = 0, fl = 0, own;
-  bool ok, first = true;
+  bool ok, first = true, agreed = false;
   // the last warp of CTA 0 (idle in thin levels) keeps the traversal's account
   const bool books = rank == 0 && wid == nw - 1;
   if (threadIdx.x == 0) link_expect(s.link, p, ncta);
@@ -871,12 +871,12 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
   for (;;) {
     // the frontier of level L - 1 is in q[p], its records in tab[p]
     ok = link_wait(s.link, p, phases, timeout_ns);
-    const LinkSum t = link_sum(s.link, p, rank, ncta);
+    const LinkSum t = link_sum<false>(s.link, p, rank, ncta);
     own = t.own;
     if (!first) {
       nf = t.x + t.y;
       mf = t.z;
-      fl = t.any ? 1u : 0u;
+      fl = t.w ? 1u : 0u;
     }
     if (!ok || nf == 0 || fl || nf > kClMaxFrontier || (uint32_t)mf > kClMaxEdges) break;
     first = false;
@@ -909,9 +909,12 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
       }
     }
     auto step = [&](const uint32_t* j, const uint32_t*, uint32_t act) { bfs_cl_push<4>(a, s, L, j, act); };
-    if (link_uneven(t, ncta)) {
+    const bool uneven = link_uneven(t, ncta);
+    if (uneven) ok = link_meet(s.link, phases, ncta, timeout_ns);
+    if (!ok) {
+      // gave up: on to the end of the step
+    } else if (uneven) {
       // redistribute: an equal slice of all entries, read from their CTAs
-      gsrb::ptx::cluster_sync();
       const uint32_t i0 = (uint32_t)((uint64_t)t.x * rank / ncta), i1 = (uint32_t)((uint64_t)t.x * (rank + 1) / ncta);
       const uint32_t gsz = cl_group(i1 - i0);
       for (uint32_t base = i0 + wid * gsz; base < i1; base += nw * gsz) {
@@ -935,7 +938,9 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
         walk_group(r.x, r.y - r.x, step);
       }
     }
-    __syncthreads();
+    agreed = true;
+    if (!(ok = link_agree(ok))) break;
+    agreed = false;
     if (wid == 0) {
       // slots (past the queue's end the entries went to the global queue), the
       // entries beyond them (less the empty slots), edges, any in the global queue
@@ -946,6 +951,8 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
     p = o;
     ++L;
   }
+  if (!agreed) ok = link_agree(ok);
+  if (!ok && threadIdx.x == 0) atomicExch(a.overflow + 1, 1u);
   if (nf == 0 || !ok) {
     if (books && lane == 0) {
       a.out[0] = L - 1;
@@ -1547,7 +1554,7 @@ __global__ void __launch_bounds__(kClThreads, 1) sssp_cluster_kernel(SsspArgs a,
   const uint32_t rank = gsrb::ptx::cluster_ctarank(), ncta = gsrb::ptx::cluster_nctarank();
   const uint32_t lane = lane_id(), wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   if (threadIdx.x == 0) {
-    link_init(s.link);
+    link_init(s.link, ncta);
     s.n[0] = s.n[1] = s.m[0] = s.m[1] = s.leave[0] = s.leave[1] = s.farn[0] = s.farn[1] = 0;
     s.fat[0] = s.fat[1] = 3u;  // nothing is known of the source
     if (rank == 0) {
@@ -1562,14 +1569,13 @@ __global__ void __launch_bounds__(kClThreads, 1) sssp_cluster_kernel(SsspArgs a,
   unsigned long long edges = 0;
   long long T = a.delta;
   const bool books = rank == 0 && wid == nw - 1;
-  bool ok, done = false;
+  bool ok, done = false, agreed = false;
   for (;;) {
     // this step's near entries are in q[p], the far pile in far[f]
     ok = link_wait(s.link, p, phases, timeout_ns);
-    const LinkSum t = link_sum(s.link, p, rank, ncta);
+    const LinkSum t = link_sum<true>(s.link, p, rank, ncta);
     own = t.own;
-    const bool leave = __any_sync(0xffffffffu, lane < ncta && s.link.tab[p][lane].w != 0u);
-    if (!ok || leave || t.x > kClMaxFrontier || t.z > kClMaxEdges) break;
+    if (!ok || t.w || t.x > kClMaxFrontier || t.z > kClMaxEdges) break;
     if (t.x == 0 && t.y == 0) {
       done = true;
       break;
@@ -1630,9 +1636,12 @@ __global__ void __launch_bounds__(kClThreads, 1) sssp_cluster_kernel(SsspArgs a,
         };
         walk_group(e.y, e.z - e.y, step);
       };
-      if (link_uneven(t, ncta)) {
+      const bool uneven = link_uneven(t, ncta);
+      if (uneven) ok = link_meet(s.link, phases, ncta, timeout_ns);
+      if (!ok) {
+        // gave up: on to the end of the step
+      } else if (uneven) {
         // redistribute: an equal slice of all entries, read from their CTAs
-        gsrb::ptx::cluster_sync();
         const uint32_t i0 = (uint32_t)((uint64_t)t.x * rank / ncta);
         const uint32_t i1 = (uint32_t)((uint64_t)t.x * (rank + 1) / ncta);
         const uint32_t gsz = cl_group(i1 - i0);
@@ -1660,7 +1669,9 @@ __global__ void __launch_bounds__(kClThreads, 1) sssp_cluster_kernel(SsspArgs a,
         relaxed = 0;
       }
     }
-    __syncthreads();
+    agreed = true;
+    if (!(ok = link_agree(ok))) break;
+    agreed = false;
     if (wid == 0) {
       if (lane == 0) {
         s.fat[p] = 0;  // every thread has read it
@@ -1671,6 +1682,8 @@ __global__ void __launch_bounds__(kClThreads, 1) sssp_cluster_kernel(SsspArgs a,
     }
     p = o;
   }
+  if (!agreed) ok = link_agree(ok);
+  if (!ok && threadIdx.x == 0) atomicExch(a.overflow + 1, 1u);
   edges = warp_sum_u64(edges + relaxed);
   if (lane == 0 && edges) atomicAdd(a.out_edges, edges);
   if (!done && ok) {
@@ -2464,7 +2477,7 @@ struct gsrb_graph {
   uint32_t* fmark = nullptr;
   LevelCounters* cnt = nullptr;
   unsigned long long* fcnt = nullptr;
-  uint32_t* flags = nullptr;  // [0] overflow, [4..8) out, [8..16) BFS single-CTA state, edges at byte 64, PageRank tickets at byte 96
+  uint32_t* flags = nullptr;  // [0] overflow, [1] a cluster's wait ran out, [4..8) out, [8..16) BFS single-CTA state, edges at byte 64, PageRank tickets at byte 96
   LevelTrace* trace = nullptr;
   uint32_t trace_cap = 0;
   float* contrib[2] = {};
@@ -2761,7 +2774,7 @@ gsrb_status_t stats_of(const gsrb_graph* G, const uint32_t* h, gsrb_traversal_st
     st->delta = G->last_delta;
   }
   if (h[0]) return GSRB_ERR_OVERFLOW;
-  if (h[7]) return GSRB_ERR_TIMEOUT;
+  if (h[7] || h[1]) return GSRB_ERR_TIMEOUT;
   return GSRB_OK;
 }
 

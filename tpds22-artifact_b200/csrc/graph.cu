@@ -3100,8 +3100,10 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
                       ? cluster_ctas(ctx, (const void*)bfs_cluster_kernel, sizeof(BfsClShared))
                       : 0;
   a.staged = ncl > 0;
+  // refused before anything is enqueued that writes the caller's array
+  gsrb_status_t st = require_coresident(ctx, fn, grid, c.threads, 0, c.cluster);
+  if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[62], ctx->stream));
-  gsrb_status_t st = GSRB_OK;
   if (!a.staged) {
     GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
     st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
@@ -3133,7 +3135,10 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
     for (uint32_t turn = thin && cluster_first ? 0u : 1u;; ++turn) {
       if (!st && turn) st = whole();
       if (!st && turn) st = cluster();
-      if (st) return st;
+      if (st) {
+        cudaStreamSynchronize(ctx->stream);  // nothing writes the caller's array after the return
+        return st;
+      }
       GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
       GSRB_CUDA(copy_status(ctx, G, 0));
       GSRB_CUDA(cudaStreamSynchronize(ctx->stream));
@@ -3207,8 +3212,10 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
   void* args[] = {&gb, &a};
   if (!ctx->events[62]) GSRB_CUDA(cudaEventCreate(&ctx->events[62]));
   if (!ctx->events[63]) GSRB_CUDA(cudaEventCreate(&ctx->events[63]));
+  // refused before anything is enqueued that writes the caller's array
+  gsrb_status_t st = require_coresident(ctx, fn, grid, c.threads, 0, c.cluster);
+  if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[62], ctx->stream));
-  gsrb_status_t st = GSRB_OK;
   if (!a.staged) {
     GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
   } else {
@@ -3220,10 +3227,12 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
     unsigned long long timeout_ns = gb.timeout_ns;
     void* cargs[] = {&a, &timeout_ns};
     st = launch_persistent(ctx, (const void*)sssp_cluster_kernel, ncl, kClThreads, sizeof(SsspClShared), ncl, 0, cargs);
-    if (st) return st;
   }
-  st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
-  if (st) return st;
+  if (!st) st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
+  if (st) {
+    cudaStreamSynchronize(ctx->stream);  // nothing writes the caller's array after the return
+    return st;
+  }
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
   st = finish_stats(ctx, G, stats);
   if (stats) stats->launch = launch;

@@ -92,6 +92,8 @@ gsrb::GridBarrier make_barrier(gsrb_ctx* ctx, const gsrb_cfg_t& c, int slot, uin
 // anything that kernel uses).
 gsrb_status_t launch_persistent(gsrb_ctx* ctx, const void* fn, int grid, int block, size_t smem,
                                 int cluster, int coop, void** args, bool pdl = false);
+// The check alone, for calls that enqueue other kernels ahead of the persistent one.
+gsrb_status_t require_coresident(gsrb_ctx* ctx, const void* fn, int grid, int block, size_t smem, int cluster);
 // Whether a plain launch is made early (programmatic serialisation, waiting for
 // the kernel before it ahead of its first access, then letting the next one in):
 // on the context's own stream, which nobody else launches on, so that the

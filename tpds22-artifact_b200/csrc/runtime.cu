@@ -170,10 +170,8 @@ static gsrb_status_t coresident_query(gsrb_ctx* ctx, const void* fn, int block, 
   return GSRB_OK;
 }
 
-gsrb_status_t launch_persistent(gsrb_ctx* ctx, const void* fn, int grid, int block, size_t smem,
-                                int cluster, int coop, void** args, bool pdl) {
+gsrb_status_t require_coresident(gsrb_ctx* ctx, const void* fn, int grid, int block, size_t smem, int cluster) {
   if (grid <= 0 || block <= 0 || block > 1024) return GSRB_ERR_ARG;
-  if (pdl && coop > 0) return GSRB_ERR_UNSUPPORTED;
   if (cluster < 1) cluster = 1;
   if (grid % cluster) return GSRB_ERR_ARG;
   int cap = 0;
@@ -185,6 +183,15 @@ gsrb_status_t launch_persistent(gsrb_ctx* ctx, const void* fn, int grid, int blo
               grid, cap, cluster);
     return GSRB_ERR_NOT_CORESIDENT;
   }
+  return GSRB_OK;
+}
+
+gsrb_status_t launch_persistent(gsrb_ctx* ctx, const void* fn, int grid, int block, size_t smem,
+                                int cluster, int coop, void** args, bool pdl) {
+  if (pdl && coop > 0) return GSRB_ERR_UNSUPPORTED;
+  if (cluster < 1) cluster = 1;
+  gsrb_status_t st = require_coresident(ctx, fn, grid, block, smem, cluster);
+  if (st) return st;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)grid, 1, 1);
   cfg.blockDim = dim3((unsigned)block, 1, 1);

@@ -364,7 +364,8 @@ gsrb_status_t gsrb_graph_is_symmetric(gsrb_graph_t g, int32_t* symmetric);
 gsrb_status_t gsrb_graph_set_policy(gsrb_graph_t g, const float* h_weights, size_t count);
 /* Two launch configurations (barrier variant, CTAs per SM, threads) for
  * learned traversals: gsrb_bfs in GSRB_BFS_LEARNED mode with cfg == NULL then
- * runs the one head 3 of the policy picks.  Both NULL: forget them. */
+ * runs its grid levels under the one head 3 of the policy picks.  Both NULL:
+ * forget them. */
 gsrb_status_t gsrb_graph_set_launch_choices(gsrb_graph_t g, const gsrb_cfg_t* cfg0, const gsrb_cfg_t* cfg1);
 /* The policy's launch choice for a BFS from src: head 3 evaluated on the host
  * on the first level's features (frontier = src); *choice = 1 if it is > 0,
@@ -373,13 +374,22 @@ gsrb_status_t gsrb_graph_policy_launch(gsrb_graph_t g, uint32_t src, int32_t* ch
 /* Copy up to max_records 48-byte per-level trace records of the last traversal. */
 gsrb_status_t gsrb_graph_trace(gsrb_graph_t g, void* h_out, uint32_t max_records, uint32_t* records);
 /* BFS levels from src into d_level (int32[n]; INT32_MAX = unreachable).
- * cfg == NULL: 2 CTAs x 512 threads per SM. */
+ * cfg: one launch of that barrier and shape for the whole traversal.
+ * cfg == NULL: the library chooses, 2 CTAs x 512 threads per SM; in
+ * GSRB_BFS_HEURISTIC and GSRB_BFS_LEARNED mode it runs levels of few vertices and
+ * edges on one thread-block cluster, in launches of its own that alternate with
+ * the grid's (trace direction 3; stats->kernel_ms then spans them all, the host's
+ * waits between them included). */
 gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t g, uint32_t src, int32_t* d_level, int32_t mode,
                        const gsrb_cfg_t* cfg, gsrb_traversal_stats_t* stats);
 /* SSSP distances (near-far buckets of width delta) into d_dist (int32[n]).
  * delta == GSRB_SSSP_DELTA_LEARNED: the graph's SSSP policy picks the width
  * (and, with cfg == NULL and launch choices set, the launch configuration);
- * GSRB_ERR_STATE without one.  The distances do not depend on either. */
+ * GSRB_ERR_STATE without one.  The distances do not depend on either.
+ * cfg: one launch of that barrier and shape for the whole traversal.  cfg ==
+ * NULL: the library chooses, 2 CTAs x 512 threads per SM; on graphs of fewer
+ * than 8 edges a vertex one thread-block cluster runs the rounds until they
+ * outgrow it (trace direction 3), and the grid the rest. */
 enum { GSRB_SSSP_DELTA_LEARNED = 0 };
 gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t g, uint32_t src, int32_t* d_dist, int32_t delta,
                         const gsrb_cfg_t* cfg, gsrb_traversal_stats_t* stats);

@@ -206,3 +206,31 @@ def test_sssp_vertices_without_out_edges(gsrb, ctx, orc, tail):
         rc, st = dg.bfs(source, out)
         gsrb.check(rc, "bfs")
         assert np.array_equal(out.download(), orc.bfs(g, source))
+
+
+@pytest.mark.parametrize("name", ["path", "wide", "tree"])
+def test_explicit_launch_runs_alone(gsrb, ctx, orc, thin_graphs, name):
+    """A launch configuration of the caller's runs the whole traversal: one
+    launch, whatever the graph; without one thin steps run on the cluster."""
+    g = thin_graphs[name]
+    dg = ctx.graph(g)
+    dg.set_policy(gsrb.mlp_init(77))
+    out = ctx.array(g.nnodes, np.int32)
+
+    def launches(call):
+        n0 = gsrb.launch_count()
+        rc, st = call()
+        gsrb.check(rc, "traversal")
+        return gsrb.launch_count() - n0
+
+    want, dist = orc.bfs(g, 0), orc.dijkstra(g, 0)
+    for variant in (gsrb.BAR_SOFT2, gsrb.BAR_FLAT, gsrb.BAR_CCG, gsrb.BAR_FANOUT):
+        c = gsrb.cfg(variant=variant, ctas_per_sm=1, threads=128, cluster=1)
+        for mode in (gsrb.BFS_HEURISTIC, gsrb.BFS_LEARNED):
+            assert launches(lambda: dg.bfs(0, out, mode, c)) == 1
+            assert np.array_equal(out.download(), want)
+        assert launches(lambda: dg.sssp(0, out, 400, c)) == 1
+        assert 3 not in dg.trace()["dir"]
+        assert np.array_equal(out.download(), dist)
+    assert launches(lambda: dg.bfs(0, out)) >= 2 and launches(lambda: dg.sssp(0, out, 400)) >= 2
+    assert np.all(dg.trace()["dir"] == 3)

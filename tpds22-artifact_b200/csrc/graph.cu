@@ -3,8 +3,9 @@
 // heuristic or by the learned policy), SSSP (near-far buckets with atomicMin)
 // and pull PageRank (FP32 state, FP64 per-vertex accumulation, fixed
 // iteration count).  One grid kernel per traversal, one grid barrier per level /
-// bucket step / iteration; thin BFS levels and thin graphs' SSSP rounds run on
-// one cluster instead (bfs_cluster_kernel, sssp_cluster_kernel).
+// bucket step / iteration; without a launch configuration of the caller's, thin
+// BFS levels and thin graphs' SSSP rounds run on one cluster instead
+// (bfs_cluster_kernel, sssp_cluster_kernel).
 //
 // Reference: the GGC "outlined iterate" kernels gg_main_pipe_1_gpu_gb of
 // LONESTAR/apps/bfs/kernel_gsrb.cu:591-626 (BFS), apps/sssp/kernel_gsrb.cu:637-687
@@ -3095,8 +3096,9 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
   void* args[] = {&gb, &a};
   if (!ctx->events[62]) GSRB_CUDA(cudaEventCreate(&ctx->events[62]));
   if (!ctx->events[63]) GSRB_CUDA(cudaEventCreate(&ctx->events[63]));
-  // The schedules that choose per level run thin levels on one cluster.
-  const int ncl = mode == GSRB_BFS_HEURISTIC || mode == GSRB_BFS_LEARNED
+  // The schedules that choose per level run thin levels on one cluster, unless
+  // the caller chose the launch: then every level runs under that.
+  const int ncl = !cfgin && (mode == GSRB_BFS_HEURISTIC || mode == GSRB_BFS_LEARNED)
                       ? cluster_ctas(ctx, (const void*)bfs_cluster_kernel, sizeof(BfsClShared))
                       : 0;
   a.staged = ncl > 0;
@@ -3202,9 +3204,10 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
   a.state = G->flags + 8;
   G->last_delta = delta;
   std::lock_guard<std::mutex> g(ctx->mu);
-  // thin graphs (mean degree < kThinDegree) start on one cluster; the grid
-  // kernel queued behind it returns at once unless the traversal outgrew it
-  const int ncl = G->m / kThinDegree < G->n
+  // thin graphs (mean degree < kThinDegree) start on one cluster, unless the
+  // caller chose the launch; the grid kernel queued behind it returns at once
+  // unless the traversal outgrew the cluster
+  const int ncl = !cfgin && G->m / kThinDegree < G->n
                       ? cluster_ctas(ctx, (const void*)sssp_cluster_kernel, sizeof(SsspClShared))
                       : 0;
   a.staged = ncl > 0;

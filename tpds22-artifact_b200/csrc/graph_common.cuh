@@ -35,7 +35,7 @@ struct DevCSR {
 // One record per level / bucket step, written by CTA 0 after the barrier.
 struct LevelTrace {
   uint32_t level;
-  uint32_t dir;          // 0 push-worklist, 1 pull, 2 push-topology, 3 push by a single CTA
+  uint32_t dir;          // 0 push-worklist, 1 pull, 2 push-topology, 3 push by a single CTA or cluster
   uint32_t nf;           // frontier vertices entering this level
   uint32_t nu;           // unvisited vertices before this level
   unsigned long long mf; // frontier out-edges

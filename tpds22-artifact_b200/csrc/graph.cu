@@ -118,7 +118,7 @@ __device__ __noinline__ void bfs_solo(const BfsArgs& a, uint32_t L, uint32_t nre
       m_acc += d;
     };
     expand_hub_ranges(one, hin, nbig, push_edge);
-    const PushSink sink{qout, hout, &s_c.n_reg, &s_c.n_big, g.n, a.overflow, nullptr, nullptr, 0u, nullptr};
+    const PushSink sink{qout, hout, &s_c.n_reg, &s_c.n_big, g.n, a.overflow, nullptr, nullptr, 0u};
     auto lanes = [&](uint32_t b, uint32_t mine, uint32_t kmax) {
       bfs_push_lanes(g, a.level, Li, b, mine, kmax, false, sink, m_acc);
     };
@@ -334,9 +334,13 @@ __device__ __forceinline__ void bfs_push_hubs(const BfsArgs& a, const Team& team
 }
 
 // The traversal body, relative to a team (the whole grid, or one instance's
-// CTA range in a batch, synchronised by `bar`).
+// CTA range in a batch, synchronised by `bar`).  a_shared: the arguments in
+// shared memory, for the single-CTA phase (a call that takes their address; of
+// the kernel's parameters that is a local copy, whose reads miss L1 after every
+// barrier, and the whole level loop would use it).
 template <int V>
-__device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const BfsArgs& a, const Team team) {
+__device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const BfsArgs& a, const BfsArgs& a_shared,
+                                        const Team team) {
   __shared__ uint32_t s_dir;
   __shared__ float s_pred;
   __shared__ MLPShared s_mlp;
@@ -489,7 +493,7 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
 
     if (!a.staged && team.ncta > 1 && dir == DIR_PUSH && nf <= blockDim.x && mf <= 4ull * blockDim.x &&
         (a.mode == GSRB_BFS_HEURISTIC || a.mode == GSRB_BFS_LEARNED)) {
-      if (team.cta == 0) bfs_solo(a, L, nreg, nbig, nu, mu, edges, prev_nf);
+      if (team.cta == 0) bfs_solo(a_shared, L, nreg, nbig, nu, mu, edges, prev_nf);
       ok = bar.sync();
       if (!ok) break;
       L = __ldcg(a.solo + 0);
@@ -512,36 +516,46 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
     // regular-queue slots reserved per warp in chunks of 64 (one counter atomic
     // per chunk) when the queue's 2n slots can hold every warp's holes
     WarpRes res{0ull, 0u, 63ull * team.nwarps() <= g.n ? 64u : 0u};
-    const bool staged = mf >= kStageMinEdges;
+    // The CTA's stage takes the entries of levels in which a warp appends a few
+    // times at most, where a reservation per warp would be an atomic each on one
+    // line: pull levels, and the walk of a hub where the next level may pull (a
+    // push level is slower on the packed queue: R-MAT-18's second 600 -> 718 us).
+    const bool hub_stage = dir == DIR_PUSH && nbig == 1 && a.symmetric && a.mode != GSRB_BFS_PUSH;
+    const bool staged = mf >= kStageMinEdges &&
+                        (dir == DIR_PULL ? g.n / (32u * kStageMaxAppends) <= team.nwarps()
+                                         : hub_stage && mf / (32u * kStageMaxAppends) <= team.nwarps());
     uint32_t real_w = 0;  // regular entries this warp appended past the stage (warp-uniform)
-    const PushSink sink{qout, hout, &c->n_reg, &c->n_big, g.n, a.overflow, &res, &real_w, 2u * g.n,
-                        staged ? &s_stage : nullptr};
+    const PushSink sink{qout, hout, &c->n_reg, &c->n_big, g.n, a.overflow, &res, &real_w, 2u * g.n};
 
-    auto discover = [&](bool disc, uint32_t v) {
-      uint2 r = make_uint2(0u, 0u);
-      if (disc) r = make_uint2(__ldg(g.row + v), __ldg(g.row + v + 1));
+    auto append = [&](bool disc, uint2 r, bool may_stage) {
       const uint32_t d = r.y - r.x;
       const bool reg1[1] = {disc && d <= kBigDegree};
-      push_append_reg<1>(reg1, &r, sink);
+      if (may_stage && staged)
+        real_w += stage_append<1>(reg1, &r, s_stage, qout, &c->n_reg, g.n, 2u * g.n, a.overflow, res, make_uint2(0u, 0u));
+      else
+        push_append_reg<1>(reg1, &r, sink);
       warp_append(disc && d > kBigDegree, r, hout, &c->n_big, g.n, a.overflow);
       m_acc += d;
     };
-    auto push_edge = [&](uint32_t, uint32_t j, bool active) {
-      uint32_t v = 0;
+    auto claim = [&](uint32_t j, bool active, bool may_stage) {
+      uint2 r = make_uint2(0u, 0u);
       bool disc = false;
       if (active) {
-        v = __ldg(g.dst + j);
+        const uint32_t v = __ldg(g.dst + j);
         if (__ldcg(a.level + v) == kInf) disc = atomicCAS(a.level + v, kInf, Li) == kInf;
+        if (disc) r = make_uint2(__ldg(g.row + v), __ldg(g.row + v + 1));
       }
-      discover(disc, v);
+      append(disc, r, may_stage);
     };
+    auto push_edge = [&](uint32_t, uint32_t j, bool active) { claim(j, active, false); };
 
     if (dir == DIR_PUSH) {
       if (nbig > 1 && nbig <= kHubList) {
         // hubs edge-balanced over the team: every CTA builds the same prefix
         bfs_push_hubs(a, team, hin, nbig, Li, sink, m_acc);
       } else {
-        expand_hub_ranges(team, hin, nbig, push_edge);
+        auto hub_edge = [&](uint32_t, uint32_t j, bool active) { claim(j, active, true); };
+        expand_hub_ranges(team, hin, nbig, hub_edge);
       }
       if (a.lb && team.ncta > 1 && mf >= kLbMinEdges) {
         // uniform across the team: every CTA takes the two extra barriers
@@ -642,20 +656,18 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
         }
         if (found) gsrb::ptx::st_relaxed_gpu_s32(a.level + v, Li);
         // the new frontier's entries: the row range is known
-        const uint32_t d = found ? deg : 0u;
-        const uint2 range = make_uint2(b, e);
-        const bool reg1[1] = {found && d <= kBigDegree};
-        push_append_reg<1>(reg1, &range, sink);
-        warp_append(found && d > kBigDegree, range, hout, &c->n_big, g.n, a.overflow);
-        m_acc += d;
+        append(found, found ? make_uint2(b, e) : make_uint2(0u, 0u), true);
       }
     }
-    // edge sums and entry counts of the new frontier; in a large level one
+    // edge sums and entry counts of the new frontier; in a staged level one
     // update per CTA (one per warp made 4736 atomics on one line of the L2:
     // R-MAT-22's first level 27.7 -> 16.3 us)
     warp_res_close(qout, 2u * g.n, res, make_uint2(0u, 0u));
     const unsigned long long ws = warp_sum_u64(m_acc);
-    if (lane_id() == 0 && ws) atomicAdd(staged ? &s_stage.msum : &c->m_next, ws);
+    if (lane_id() == 0 && ws) {
+      if (staged) atomicAdd(&s_stage.msum, ws);
+      else atomicAdd(&c->m_next, ws);
+    }
     if (lane_id() == 0 && real_w) atomicAdd(&c->n_real, (unsigned long long)real_w);
     if (staged) stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, &c->n_real, &c->m_next);
     ok = bar.sync();
@@ -992,11 +1004,13 @@ constexpr int kGraphMaxThreads = 1024;
 
 template <int V>
 __global__ void __launch_bounds__(kGraphMaxThreads)
-bfs_kernel(gsrb::GridBarrier gb, BfsArgs a) {
+bfs_kernel(const __grid_constant__ gsrb::GridBarrier gb, const __grid_constant__ BfsArgs a) {
   __shared__ gsrb::BarrierShared bsh;
+  __shared__ BfsArgs s_args;
+  if (threadIdx.x == 0) s_args = a;  // read after the first level's barrier
   gsrb::GridSync<V> bar;
   const bool ok = bar.init(gb, &bsh);
-  bfs_run<V>(bar, ok, a, Team{blockIdx.x, gridDim.x});
+  bfs_run<V>(bar, ok, a, s_args, Team{blockIdx.x, gridDim.x});
   bar.finish();
 }
 
@@ -1760,7 +1774,7 @@ batch_kernel(const BatchDesc* __restrict__ descs, const uint16_t* __restrict__ c
   const Team team{blockIdx.x - d.first, d.count};
   gsrb::GridSync<V> bar;
   const bool ok = bar.init(d.gb, &bsh);
-  if (KIND == 0) bfs_run<V>(bar, ok, d.bfs, team);
+  if (KIND == 0) bfs_run<V>(bar, ok, d.bfs, d.bfs, team);
   else sssp_run<V>(bar, ok, d.sssp, team);
   bar.finish();
 }

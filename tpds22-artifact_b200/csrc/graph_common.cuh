@@ -384,18 +384,13 @@ struct PushSink {
   WarpRes* res;                // regular-queue reservation (null: append directly)
   uint32_t* real;              // regular entries this warp appended past the stage (with res)
   uint32_t rcap;               // regular-queue slots (with res)
-  BfsStage* stage;             // the CTA's stage (null: small level)
 };
 
-// Appends the regular entries of a push step: to the CTA's stage, through the
-// warp's reservation (small levels; both count the entries that went past the
-// stage), or directly in the single-CTA phase.
+// Appends the regular entries of a push step: through the warp's reservation
+// when there is one (counting the entries), else directly.
 template <int K>
 __device__ __forceinline__ void push_append_reg(const bool* reg, const uint2* rg, const PushSink& s) {
-  if (s.stage) {
-    *s.real += stage_append<K>(reg, rg, *s.stage, s.qout, s.n_reg, s.cap, s.rcap, s.overflow, *s.res,
-                               make_uint2(0u, 0u));
-  } else if (s.res && s.res->chunk) {
+  if (s.res && s.res->chunk) {
     *s.real += warp_append_res<K>(reg, rg, s.qout, s.n_reg, s.rcap, s.overflow, *s.res, make_uint2(0u, 0u));
   } else {
     if (s.real) {
@@ -408,10 +403,14 @@ __device__ __forceinline__ void push_append_reg(const bool* reg, const uint2* rg
   }
 }
 
-// Levels with at least this many frontier edges collect their entries in the
+// Levels with at least this many frontier edges may collect their entries in the
 // CTAs' stages; in smaller ones a warp appends about once, and the flush at the
 // level's end would only add a trip (2048^2 grid: 44.1 ms staged, 41.1 not).
+// Nor do levels in which a warp appends more often than kStageMaxAppends: its
+// reservation then costs an atomic every 64 entries, the stage one in shared
+// memory on every append.
 constexpr unsigned long long kStageMinEdges = 16384;
+constexpr uint32_t kStageMaxAppends = 4;
 
 // Frontiers up to this size check a destination's level only through the
 // claim itself (compare-and-swap INF -> L) and load its row range alongside

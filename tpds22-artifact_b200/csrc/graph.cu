@@ -1044,6 +1044,11 @@ struct SsspArgs {
 constexpr uint32_t kSsspBig = 256;
 constexpr uint32_t kSsspStep = 2;         // the grid's first step after the cluster (queue parity, counter set, stamp)
 constexpr uint32_t kProbeMeanDegree = 8;  // graphs of this mean degree probe before claiming in every round
+// Larger rounds probe on other graphs too: what they relax may be one vertex's
+// in-edges, whose claims take turns (a round of 14,500 vertices with a common
+// neighbour 14.0 us for 6.6; at 4096, which rounds of a 2048^2 grid reach, that
+// grid takes 41.3 ms for 40.0).
+constexpr uint32_t kRelaxPrecheckFrontier = 8192;
 
 // Where an SSSP relax step puts the vertices whose distance it lowered.
 struct RelaxSink {
@@ -1303,7 +1308,7 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
     // can hold the holes of every warp
     WarpRes res{0ull, 0u, 63ull * team.nwarps() <= g.n ? 64u : 0u};
     const RelaxSink sink{qout, hout, &c->n_reg, &c->n_big, fout, fc, stamp, fgen, (int32_t)min(T, (long long)kInf), &s_stage, &res, 2u * g.n,
-                         probe || nf > kPushPrecheckFrontier};
+                         probe || nf > kRelaxPrecheckFrontier};
     // vertex lists relaxed edge-balanced: edge prefix, first edge, distance
     ListSmem& L_ = list_smem();
     uint32_t* s_lp = L_.p;

@@ -53,6 +53,7 @@ struct BfsArgs {
   uint32_t* lb_part;   // [kLbMaxCtas] per-CTA edge totals
   uint32_t* phase;     // [0] PHASE_*, [1] policy decisions, [2] fallback level so far
   bool staged;         // init kernel, then cluster and grid kernels in turn (a.phase says whose turn it is)
+  bool stage;          // the launch has the CTAs' stages
 };
 
 // Whose turn it is in a traversal that alternates between one cluster (thin
@@ -344,10 +345,9 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
   __shared__ uint32_t s_dir;
   __shared__ float s_pred;
   __shared__ MLPShared s_mlp;
-  __shared__ BfsStage s_stage;
   const DevCSR& g = a.g;
   const uint32_t tid = team.tid(), nthreads = team.nthreads();
-  if (threadIdx.x == 0) stage_reset(s_stage);
+  BfsStage* const stage = cta_stage<BfsStage>(a.stage);
   if (a.mode == GSRB_BFS_LEARNED) mlp_stage(a.mlp, &s_mlp);  // visible after the barrier below
 
   uint32_t nu, prev_nf = 1, L = 1, decisions = 0;
@@ -521,7 +521,7 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
     // line: pull levels, and the walk of a hub where the next level may pull (a
     // push level is slower on the packed queue: R-MAT-18's second 600 -> 718 us).
     const bool hub_stage = dir == DIR_PUSH && nbig == 1 && a.symmetric && a.mode != GSRB_BFS_PUSH;
-    const bool staged = mf >= kStageMinEdges &&
+    const bool staged = a.stage && mf >= kStageMinEdges &&
                         (dir == DIR_PULL ? g.n / (32u * kStageMaxAppends) <= team.nwarps()
                                          : hub_stage && mf / (32u * kStageMaxAppends) <= team.nwarps());
     uint32_t real_w = 0;  // regular entries this warp appended past the stage (warp-uniform)
@@ -531,7 +531,7 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
       const uint32_t d = r.y - r.x;
       const bool reg1[1] = {disc && d <= kBigDegree};
       if (may_stage && staged)
-        real_w += stage_append<1>(reg1, &r, s_stage, qout, &c->n_reg, g.n, 2u * g.n, a.overflow, res, make_uint2(0u, 0u));
+        real_w += stage_append<1>(reg1, &r, stage, qout, &c->n_reg, g.n, 2u * g.n, a.overflow, res, make_uint2(0u, 0u));
       else
         push_append_reg<1>(reg1, &r, sink);
       warp_append(disc && d > kBigDegree, r, hout, &c->n_big, g.n, a.overflow);
@@ -665,11 +665,11 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
     warp_res_close(qout, 2u * g.n, res, make_uint2(0u, 0u));
     const unsigned long long ws = warp_sum_u64(m_acc);
     if (lane_id() == 0 && ws) {
-      if (staged) atomicAdd(&s_stage.msum, ws);
+      if (staged) atomicAdd(&stage->msum, ws);
       else atomicAdd(&c->m_next, ws);
     }
     if (lane_id() == 0 && real_w) atomicAdd(&c->n_real, (unsigned long long)real_w);
-    if (staged) stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, &c->n_real, &c->m_next);
+    if (staged) stage_flush(*stage, qout, &c->n_reg, 2u * g.n, a.overflow, &c->n_real, &c->m_next);
     ok = bar.sync();
   }
   if (to_cluster) return;
@@ -1035,6 +1035,7 @@ struct SsspArgs {
   uint32_t* phase;      // [0] PHASE_*
   uint32_t* state;      // where the cluster left off: [0] rounds, [1] buckets, [2..3] near threshold
   bool staged;          // init and cluster kernels before the grid kernel (a.phase says whether it has work)
+  bool stage;           // the launch has the CTAs' stages
 };
 
 // Vertices of more edges than this go to the near hub queue and are relaxed
@@ -1061,7 +1062,7 @@ struct RelaxSink {
   uint32_t stamp;               // near-queue stamp of this round
   uint32_t fgen;                // far-pile generation
   int32_t T;                    // near threshold (at most kInf, which no queued distance reaches)
-  IdStage* stage;               // the CTA's near-queue entries
+  IdStage* stage;               // the CTA's near-queue entries (null: none)
   WarpRes* res;                 // the warp's near-queue reservation (past the stage)
   uint32_t near_cap;            // near-queue capacity in slots (holes included)
   bool precheck;                // read a distance before claiming it (large rounds)
@@ -1152,7 +1153,7 @@ __device__ __forceinline__ void sssp_relax4e(const SsspArgs& a, const int32_t* d
     reg[r] = to_near[r] && d[r] <= kSsspBig;
     big[r] = to_near[r] && d[r] > kSsspBig;
   }
-  stage_append<4>(reg, v, *s.stage, s.qout, s.n_reg, g.n, s.near_cap, a.overflow, *s.res, kHole);
+  stage_append<4>(reg, v, s.stage, s.qout, s.n_reg, g.n, s.near_cap, a.overflow, *s.res, kHole);
   warp_append_k<4>(big, v, s.hout, s.n_big, g.n, a.overflow);
   warp_append_k<4>(to_far, v, s.fout, s.fc, g.n, a.overflow);
 }
@@ -1189,8 +1190,7 @@ template <int V>
 __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const SsspArgs& a, const Team team) {
   const DevCSR& g = a.g;
   const uint32_t tid = team.tid(), nthreads = team.nthreads();
-  __shared__ IdStage s_stage;
-  if (threadIdx.x == 0) stage_reset(s_stage);
+  IdStage* const stage = cta_stage<IdStage>(a.stage);
   uint32_t step = 1;       // index of the near counter set in use (rotating by 3)
   uint32_t rounds = 0, buckets = 1;
   // near threshold: vertices with dist < T are relaxed in the current bucket
@@ -1307,7 +1307,7 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
     // near-queue reservations in chunks of 64 slots when the queue (2n slots)
     // can hold the holes of every warp
     WarpRes res{0ull, 0u, 63ull * team.nwarps() <= g.n ? 64u : 0u};
-    const RelaxSink sink{qout, hout, &c->n_reg, &c->n_big, fout, fc, stamp, fgen, (int32_t)min(T, (long long)kInf), &s_stage, &res, 2u * g.n,
+    const RelaxSink sink{qout, hout, &c->n_reg, &c->n_big, fout, fc, stamp, fgen, (int32_t)min(T, (long long)kInf), stage, &res, 2u * g.n,
                          probe || nf > kRelaxPrecheckFrontier};
     // vertex lists relaxed edge-balanced: edge prefix, first edge, distance
     ListSmem& L_ = list_smem();
@@ -1373,7 +1373,7 @@ __device__ __forceinline__ void sssp_run(gsrb::GridSync<V>& bar, bool ok, const 
       }
     }
     warp_res_close(qout, 2u * g.n, res, kHole);
-    stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
+    if (stage) stage_flush(*stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
     relaxed_edges += my_edges;
     ++step;
     ok = bar.sync();
@@ -2041,6 +2041,7 @@ struct PrrArgs {
   unsigned long long* out_edges;
   PullArgs pull;
   bool symmetric;       // rows are also in-edge lists: rounds with many edges may pull
+  bool stage;           // the launch has the CTAs' stages
 };
 
 // A round whose worklist holds at least 1 / kPrrDense of the edges is pulled on
@@ -2065,7 +2066,7 @@ struct PrrSink {
   unsigned long long* n_reg;
   unsigned long long* n_big;
   uint32_t stamp;  // a vertex enters the next worklist at most once per round
-  IdStage* stage;  // the CTA's worklist entries
+  IdStage* stage;  // the CTA's worklist entries (null: none)
   WarpRes* res;    // the warp's worklist reservation (past the stage)
 };
 
@@ -2114,7 +2115,7 @@ __device__ __forceinline__ void prr_push4e(const PrrArgs& a, const float* upd, c
     pushes += cross[r] ? 1u : 0u;
     medges += d;
   }
-  stage_append<4>(reg, w, *s.stage, s.qout, s.n_reg, g.n, 2u * g.n, a.overflow, *s.res, kHole);
+  stage_append<4>(reg, w, s.stage, s.qout, s.n_reg, g.n, 2u * g.n, a.overflow, *s.res, kHole);
   warp_append_k<4>(big, w, s.hout, s.n_big, g.n, a.overflow);
 }
 
@@ -2156,8 +2157,7 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
   const Team team{blockIdx.x, gridDim.x};
   const uint32_t tid = team.tid(), nthreads = team.nthreads();
   const uint32_t lane = lane_id();
-  __shared__ IdStage s_stage;
-  if (threadIdx.x == 0) stage_reset(s_stage);
+  IdStage* const stage = cta_stage<IdStage>(a.stage);
   // init_1
   for (uint32_t v = tid; v < g.n; v += nthreads) {
     a.p[v] = 1.f - a.alpha;
@@ -2287,10 +2287,10 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
           const bool reg[1] = {in && d <= kBigDegree};
           const uint32_t vv[1] = {v};
           WarpRes none{0ull, 0u, 0u};
-          stage_append<1>(reg, vv, s_stage, qout, &c->n_reg, g.n, 2u * g.n, a.overflow, none, kHole);
+          stage_append<1>(reg, vv, stage, qout, &c->n_reg, g.n, 2u * g.n, a.overflow, none, kHole);
           warp_append(in && d > kBigDegree, v, hout, &c->n_big, g.n, a.overflow);
         }
-        stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
+        if (stage) stage_flush(*stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
         ok = bar.sync();
         if (!ok) break;
       }
@@ -2322,7 +2322,7 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
     // worklist reservations in chunks of 64 slots when the queue (2n slots)
     // can hold the holes of every warp (see WarpRes)
     WarpRes wres{0ull, 0u, 63ull * (nthreads >> 5) <= g.n ? 64u : 0u};
-    const PrrSink sink{qout, hout, &c->n_reg, &c->n_big, stamp, &s_stage, &wres};
+    const PrrSink sink{qout, hout, &c->n_reg, &c->n_big, stamp, stage, &wres};
     ListSmem& L_ = list_smem();
     // builds an edge-balanced list from vertex ids and their updates (CTA-wide)
     auto build_list = [&](auto id_of, auto upd_of, uint32_t cnt) {
@@ -2423,7 +2423,8 @@ pr_residual_kernel(gsrb::GridBarrier gb, PrrArgs a) {
     warp_res_close(qout, 2u * g.n, wres, kHole);
     medges = warp_sum_u64(medges);
     if (lane == 0 && medges) atomicAdd(&s_edges, medges);
-    stage_flush(s_stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
+    if (stage) stage_flush(*stage, qout, &c->n_reg, 2u * g.n, a.overflow, nullptr, nullptr);
+    else __syncthreads();
     if (threadIdx.x == 0 && s_edges) atomicAdd(&c->m_next, s_edges);
     ok = bar.sync();
     if (!ok) break;
@@ -2767,6 +2768,17 @@ PullArgs pull_args(const gsrb_graph* G, const gsrb_cfg_t& c) {
   a.ticket = reinterpret_cast<unsigned long long*>(G->flags + 24);
   a.gather_l1 = c.form == GSRB_FORM_L2 ? 0 : 1;
   return a;
+}
+
+// Dynamic shared memory of a launch: the CTAs' stages where the grid is co-resident
+// with them, else none (8 x 128 threads per SM fit without; the kernel then
+// appends through the warps' reservations).
+template <class S>
+size_t with_stage(gsrb_ctx* ctx, const void* fn, int grid, const gsrb_cfg_t& c, int cluster) {
+  int cap = 0;
+  return coresident_ctas(ctx, fn, c.threads, sizeof(S), cluster < 1 ? 1 : cluster, &cap) == GSRB_OK && cap >= grid
+             ? sizeof(S)
+             : 0;
 }
 
 // CTAs of the cluster that runs thin steps: 16, 8 where 16 cannot be placed,
@@ -3124,10 +3136,12 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
   // refused before anything is enqueued that writes the caller's array
   gsrb_status_t st = require_coresident(ctx, fn, grid, c.threads, 0, c.cluster);
   if (st) return st;
+  const size_t smem = with_stage<BfsStage>(ctx, fn, grid, c, c.cluster);
+  a.stage = smem != 0;
   GSRB_CUDA(cudaEventRecord(ctx->events[62], ctx->stream));
   if (!a.staged) {
     GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
-    st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
+    st = launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop_of(c), args);
     if (st) return st;
     GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
   } else {
@@ -3145,7 +3159,7 @@ gsrb_status_t gsrb_bfs(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d_
       return launch_persistent(ctx, (const void*)bfs_cluster_kernel, ncl, kClThreads, sizeof(BfsClShared), ncl, 0,
                                cargs);
     };
-    auto whole = [&] { return launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args); };
+    auto whole = [&] { return launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop_of(c), args); };
     // A kernel whose turn it is not returns at once, so the usual order is
     // queued without a look at the device: the cluster for the whole of a thin
     // graph; cluster, grid and the thin last levels on the cluster again
@@ -3237,6 +3251,8 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
   // refused before anything is enqueued that writes the caller's array
   gsrb_status_t st = require_coresident(ctx, fn, grid, c.threads, 0, c.cluster);
   if (st) return st;
+  const size_t smem = with_stage<IdStage>(ctx, fn, grid, c, c.cluster);
+  a.stage = smem != 0;
   GSRB_CUDA(cudaEventRecord(ctx->events[62], ctx->stream));
   if (!a.staged) {
     GSRB_CUDA(cudaMemsetAsync(G->flags, 0, 128, ctx->stream));
@@ -3250,7 +3266,7 @@ gsrb_status_t gsrb_sssp(gsrb_ctx_t ctx, gsrb_graph_t G, uint32_t src, int32_t* d
     void* cargs[] = {&a, &timeout_ns};
     st = launch_persistent(ctx, (const void*)sssp_cluster_kernel, ncl, kClThreads, sizeof(SsspClShared), ncl, 0, cargs);
   }
-  if (!st) st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
+  if (!st) st = launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop_of(c), args);
   if (st) {
     cudaStreamSynchronize(ctx->stream);  // nothing writes the caller's array after the return
     return st;
@@ -3311,6 +3327,8 @@ gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha
   a.p = d_rank;
   a.pull = pull_args(G, c);
   a.symmetric = G->symmetric;
+  const size_t smem = with_stage<IdStage>(ctx, fn, grid, c, c.cluster);
+  a.stage = smem != 0;
   a.r = G->contrib[0];
   a.hub_upd = G->contrib[1];
   a.mark = G->mark;
@@ -3331,7 +3349,7 @@ gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t G, float alpha
   if (!ctx->events[62]) GSRB_CUDA(cudaEventCreate(&ctx->events[62]));
   if (!ctx->events[63]) GSRB_CUDA(cudaEventCreate(&ctx->events[63]));
   GSRB_CUDA(cudaEventRecord(ctx->events[62], ctx->stream));
-  gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, 0, c.cluster, coop_of(c), args);
+  gsrb_status_t st = launch_persistent(ctx, fn, grid, c.threads, smem, c.cluster, coop_of(c), args);
   if (st) return st;
   GSRB_CUDA(cudaEventRecord(ctx->events[63], ctx->stream));
   return finish_stats(ctx, G, stats);
@@ -3354,7 +3372,7 @@ struct gsrb_batch {
 
 namespace {
 
-BfsArgs bfs_args(gsrb_graph* G, uint32_t src, int32_t* level, int32_t mode) {
+BfsArgs bfs_args(gsrb_graph* G, uint32_t src, int32_t* level, int32_t mode, bool stage) {
   BfsArgs a;
   a.g = dev_csr(G);
   a.src = src;
@@ -3381,10 +3399,11 @@ BfsArgs bfs_args(gsrb_graph* G, uint32_t src, int32_t* level, int32_t mode) {
   a.lb_part = G->lb_part;
   a.phase = G->flags + 20;
   a.staged = false;
+  a.stage = stage;
   return a;
 }
 
-SsspArgs sssp_args(gsrb_graph* G, uint32_t src, int32_t* dist, int32_t delta) {
+SsspArgs sssp_args(gsrb_graph* G, uint32_t src, int32_t* dist, int32_t delta, bool stage) {
   SsspArgs a;
   a.g = dev_csr(G);
   a.src = src;
@@ -3407,6 +3426,7 @@ SsspArgs sssp_args(gsrb_graph* G, uint32_t src, int32_t* dist, int32_t delta) {
   a.phase = G->flags + 20;
   a.state = G->flags + 8;
   a.staged = false;
+  a.stage = stage;
   return a;
 }
 
@@ -3430,6 +3450,8 @@ gsrb_status_t batch_launch(gsrb_batch* B, const uint32_t* srcs, int32_t* const* 
   const void* fn = batch_fn(B->cfg.variant, kind);
   if (!fn) return GSRB_ERR_UNSUPPORTED;
   std::lock_guard<std::mutex> g(ctx->mu);
+  const size_t smem = kind == 0 ? with_stage<BfsStage>(ctx, fn, B->grid, B->cfg, 1)
+                                : with_stage<IdStage>(ctx, fn, B->grid, B->cfg, 1);
   std::vector<BatchDesc> desc((size_t)k);
   for (int i = 0; i < k; ++i) {
     BatchDesc& d = desc[i];
@@ -3441,11 +3463,11 @@ gsrb_status_t batch_launch(gsrb_batch* B, const uint32_t* srcs, int32_t* const* 
     d.count = B->count[i];
     d.kind = (uint32_t)kind;
     if (kind == 0) {
-      d.bfs = bfs_args(B->graphs[i], srcs[i], outs[i], param);
+      d.bfs = bfs_args(B->graphs[i], srcs[i], outs[i], param, smem != 0);
       B->graphs[i]->last_delta = 0;
     }
     else {
-      d.sssp = sssp_args(B->graphs[i], srcs[i], outs[i], deltas[i]);
+      d.sssp = sssp_args(B->graphs[i], srcs[i], outs[i], deltas[i], smem != 0);
       B->graphs[i]->last_delta = deltas[i];
     }
     GSRB_CUDA(cudaMemsetAsync(B->graphs[i]->flags, 0, 128, ctx->stream));
@@ -3466,7 +3488,7 @@ gsrb_status_t batch_launch(gsrb_batch* B, const uint32_t* srcs, int32_t* const* 
   const BatchDesc* dd = B->d_desc;
   const uint16_t* ci = B->d_cta_inst;
   void* args[] = {(void*)&dd, (void*)&ci};
-  return launch_persistent(ctx, fn, B->grid, B->cfg.threads, 0, 1, coop_of(B->cfg), args);
+  return launch_persistent(ctx, fn, B->grid, B->cfg.threads, smem, 1, coop_of(B->cfg), args);
 }
 
 }  // namespace

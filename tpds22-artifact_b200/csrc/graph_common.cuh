@@ -185,7 +185,8 @@ __device__ __forceinline__ void warp_res_close(T* q, uint32_t cap, WarpRes& res,
 // to the queue at the round's end with one reservation on the shared counter
 // (stage_flush): an append costs a shared-memory atomic instead of a trip to
 // the L2, and the queue has no holes.  A round that outgrows the stage appends
-// the rest through the warps' reservations.
+// the rest through the warps' reservations.  The stage is the kernels' dynamic
+// shared memory: a launch has one where its CTAs fit with it (see with_stage).
 template <class T, uint32_t CAP>
 struct Stage {
   static constexpr uint32_t kCap = CAP;
@@ -204,9 +205,10 @@ __device__ __forceinline__ void stage_reset(Stage<T, CAP>& st) {  // thread 0, b
   st.msum = 0;
 }
 
-// Returns the number of entries that went past the stage.  Warp-synchronous.
+// Returns the number of entries that went past the stage (all where there is
+// none, unless a reservation takes and counts them).  Warp-synchronous.
 template <int K, class T, uint32_t CAP>
-__device__ __forceinline__ uint32_t stage_append(const bool* pred, const T* v, Stage<T, CAP>& st, T* q,
+__device__ __forceinline__ uint32_t stage_append(const bool* pred, const T* v, Stage<T, CAP>* st, T* q,
                                                  unsigned long long* cnt, uint32_t cap, uint32_t res_cap,
                                                  uint32_t* overflow, WarpRes& res, T hole) {
   uint32_t mask[K];
@@ -217,20 +219,22 @@ __device__ __forceinline__ uint32_t stage_append(const bool* pred, const T* v, S
     tot += __popc(mask[r]);
   }
   if (!tot) return 0;
-  uint32_t pos = 0;
-  if (lane_id() == 0) {
-    pos = atomicAdd(&st.n, tot);
-    if (pos + tot > CAP) atomicMin(&st.limit, pos);
-  }
-  pos = __shfl_sync(0xffffffffu, pos, 0);
-  if (pos + tot <= CAP) {
-    const uint32_t lt = lanemask_lt();
-#pragma unroll
-    for (int r = 0; r < K; ++r) {
-      if (pred[r]) st.buf[pos + __popc(mask[r] & lt)] = v[r];
-      pos += __popc(mask[r]);
+  if (st) {
+    uint32_t pos = 0;
+    if (lane_id() == 0) {
+      pos = atomicAdd(&st->n, tot);
+      if (pos + tot > CAP) atomicMin(&st->limit, pos);
     }
-    return 0;
+    pos = __shfl_sync(0xffffffffu, pos, 0);
+    if (pos + tot <= CAP) {
+      const uint32_t lt = lanemask_lt();
+#pragma unroll
+      for (int r = 0; r < K; ++r) {
+        if (pred[r]) st->buf[pos + __popc(mask[r] & lt)] = v[r];
+        pos += __popc(mask[r]);
+      }
+      return 0;
+    }
   }
   if (res.chunk) return warp_append_res<K>(pred, v, q, cnt, res_cap, overflow, res, hole);
   warp_append_k<K>(pred, v, q, cnt, cap, overflow);
@@ -264,6 +268,16 @@ __device__ __forceinline__ void stage_flush(Stage<T, CAP>& st, T* q, unsigned lo
 constexpr uint32_t kBfsStage = 2048, kIdStage = 4096;
 using BfsStage = Stage<uint2, kBfsStage>;
 using IdStage = Stage<uint32_t, kIdStage>;
+
+// The CTA's stage, empty after the next CTA barrier; null in a launch without one.
+extern __shared__ __align__(16) unsigned char stage_smem[];
+template <class S>
+__device__ __forceinline__ S* cta_stage(bool have) {
+  if (!have) return nullptr;
+  S* st = reinterpret_cast<S*>(stage_smem);
+  if (threadIdx.x == 0) stage_reset(*st);
+  return st;
+}
 
 __device__ __forceinline__ unsigned long long warp_sum_u64(unsigned long long v) {
 #pragma unroll

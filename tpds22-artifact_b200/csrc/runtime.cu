@@ -138,12 +138,14 @@ static gsrb_status_t coresident_query(gsrb_ctx* ctx, const void* fn, int block, 
   // raise the kernel's dynamic shared-memory limit to what the device allows
   // next to the kernel's static shared memory (a limit set to this launch's
   // size could be below a later, cached shape's)
-  if (smem > 32 * 1024) {  // (static shared memory counts towards the 48 KiB too)
+  if (smem > 0) {
     cudaFuncAttributes fa;
     GSRB_CUDA(cudaFuncGetAttributes(&fa, fn));
-    int lim = ctx->max_smem_optin - (int)fa.sharedSizeBytes;
-    if (lim < (int)smem) lim = (int)smem;  // too large: the call below reports it
-    GSRB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    if (fa.sharedSizeBytes + smem > 48 * 1024) {  // (static shared memory counts towards the 48 KiB too)
+      int lim = ctx->max_smem_optin - (int)fa.sharedSizeBytes;
+      if (lim < (int)smem) lim = (int)smem;  // too large: the call below reports it
+      GSRB_CUDA(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, lim));
+    }
   }
   if (cluster <= 1) {
     int nb = 0;

@@ -439,7 +439,9 @@ gsrb_status_t gsrb_pagerank_residual(gsrb_ctx_t ctx, gsrb_graph_t g, float alpha
  * sub-grid barrier of its own carved from the context's barrier state, so
  * instances never wait for each other.  cfg->variant must not use hardware
  * cluster barriers (SOFT2, FLAT, TREE, FLIP, FANOUT; default FANOUT).
- * The launches are asynchronous and can be captured in a CUDA graph. */
+ * The launches are asynchronous and can be captured in a CUDA graph: a replay
+ * runs the sources and arrays of the captured call, whatever was called since
+ * (each captured call keeps a descriptor block until the batch is freed). */
 typedef struct gsrb_batch* gsrb_batch_t;
 gsrb_status_t gsrb_batch_create(gsrb_ctx_t ctx, const gsrb_graph_t* graphs, int32_t k, const gsrb_cfg_t* cfg,
                                 gsrb_batch_t* out);

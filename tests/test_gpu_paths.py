@@ -234,3 +234,60 @@ def test_explicit_launch_runs_alone(gsrb, ctx, orc, thin_graphs, name):
         assert np.array_equal(out.download(), dist)
     assert launches(lambda: dg.bfs(0, out)) >= 2 and launches(lambda: dg.sssp(0, out, 400)) >= 2
     assert np.all(dg.trace()["dir"] == 3)
+
+
+def test_batch_replay_between_live_calls(gsrb, ctx, orc, path_graphs):
+    """A replay runs the captured call, whatever ran live before the capture,
+    between it and the replay, or is enqueued right behind the replay."""
+    gs = [path_graphs["grid"], path_graphs["degrees"]]
+    dgs = [ctx.graph(g) for g in gs]
+    b = gsrb.Batch(ctx, dgs)
+    outs = {k: [ctx.array(g.nnodes, np.int32) for g in gs] for k in ("live", "bfs", "sssp")}
+
+    def live(src):
+        gsrb.check(b.bfs([src] * 2, outs["live"], gsrb.BFS_PUSH), "live")
+
+    def holds(key, f):
+        for g, o in zip(gs, outs[key]):
+            assert np.array_equal(o.download(), f(g))
+
+    live(3)
+    execs = []
+    for key in ("bfs", "sssp"):  # two captured calls on one batch
+        cg = gsrb.CudaGraph(ctx)
+        with cg:
+            gsrb.check(b.bfs([7] * 2, outs[key]) if key == "bfs" else b.sssp([9] * 2, outs[key], 500), "captured")
+        execs.append(cg)
+    live(11)
+    for _ in range(3):
+        for key in ("bfs", "sssp"):
+            for o in outs[key]:
+                o.zero()
+        live(5)
+        execs[0].launch()
+        live(12)
+        execs[1].launch()
+        live(13)
+        gsrb.check(b.stats()[0], "stats")
+        holds("bfs", lambda g: orc.bfs(g, 7))
+        holds("sssp", lambda g: orc.dijkstra(g, 9))
+        holds("live", lambda g: orc.bfs(g, 13))
+    for cg in execs:
+        cg.free()
+    b.free()
+
+
+def test_batch_first_call_captured(gsrb, ctx, orc, path_graphs):
+    """The first call on a batch, of a shape not launched before, may be a captured one."""
+    gs = [path_graphs["grid"], path_graphs["rmat"]]
+    outs = [ctx.array(g.nnodes, np.int32) for g in gs]
+    b = gsrb.Batch(ctx, [ctx.graph(g) for g in gs], gsrb.cfg(variant=gsrb.BAR_FLIP, ctas_per_sm=1, threads=352))
+    cg = gsrb.CudaGraph(ctx)
+    with cg:
+        gsrb.check(b.sssp([4] * 2, outs, 700), "captured")
+    cg.launch()
+    gsrb.check(b.stats()[0], "stats")
+    for g, o in zip(gs, outs):
+        assert np.array_equal(o.download(), orc.dijkstra(g, 4))
+    cg.free()
+    b.free()

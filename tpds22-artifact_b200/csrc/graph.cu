@@ -3364,8 +3364,11 @@ struct gsrb_batch {
   gsrb_cfg_t cfg;
   int grid = 0;
   std::vector<uint32_t> first, count;
-  BatchDesc* h_desc = nullptr;  // pinned; read by the last call's copy until `copied`
+  BatchDesc* h_desc = nullptr;  // pinned; read by the last live call's copy until `copied`
   cudaEvent_t copied = nullptr;
+  // A captured call's copy reads its source at every replay, so each has a
+  // pinned block of its own, kept until the batch is freed.
+  std::vector<BatchDesc*> h_captured;
   BatchDesc* d_desc = nullptr;
   uint16_t* d_cta_inst = nullptr;
 };
@@ -3470,17 +3473,28 @@ gsrb_status_t batch_launch(gsrb_batch* B, const uint32_t* srcs, int32_t* const* 
       d.sssp = sssp_args(B->graphs[i], srcs[i], outs[i], deltas[i], smem != 0);
       B->graphs[i]->last_delta = deltas[i];
     }
-    GSRB_CUDA(cudaMemsetAsync(B->graphs[i]->flags, 0, 128, ctx->stream));
   }
-  // The copy of an earlier call may not have run yet (calls are asynchronous):
-  // its source is rewritten only when the descriptors differ, and after it.
-  if (memcmp(B->h_desc, desc.data(), sizeof(BatchDesc) * (size_t)k) != 0) {
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  GSRB_CUDA(cudaStreamIsCapturing(ctx->stream, &capturing));
+  const BatchDesc* src = B->h_desc;
+  if (capturing != cudaStreamCaptureStatusNone) {
+    BatchDesc* block = nullptr;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;  // (an allocation is not part of what is recorded)
+    GSRB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    const cudaError_t e = cudaMallocHost(&block, sizeof(BatchDesc) * (size_t)k);
+    GSRB_CUDA(cudaThreadExchangeStreamCaptureMode(&mode));
+    GSRB_CUDA(e);
+    B->h_captured.push_back(block);
+    memcpy(block, desc.data(), sizeof(BatchDesc) * (size_t)k);
+    src = block;
+  } else if (memcmp(B->h_desc, desc.data(), sizeof(BatchDesc) * (size_t)k) != 0) {
+    // The copy of an earlier call may not have run yet (calls are asynchronous):
+    // its source is rewritten only when the descriptors differ, and after it.
     if (B->copied) GSRB_CUDA(cudaEventSynchronize(B->copied));
     memcpy(B->h_desc, desc.data(), sizeof(BatchDesc) * (size_t)k);
   }
-  GSRB_CUDA(cudaMemcpyAsync(B->d_desc, B->h_desc, sizeof(BatchDesc) * k, cudaMemcpyHostToDevice, ctx->stream));
-  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
-  GSRB_CUDA(cudaStreamIsCapturing(ctx->stream, &capturing));
+  for (int i = 0; i < k; ++i) GSRB_CUDA(cudaMemsetAsync(B->graphs[i]->flags, 0, 128, ctx->stream));
+  GSRB_CUDA(cudaMemcpyAsync(B->d_desc, src, sizeof(BatchDesc) * k, cudaMemcpyHostToDevice, ctx->stream));
   if (capturing == cudaStreamCaptureStatusNone) {
     if (!B->copied) GSRB_CUDA(cudaEventCreateWithFlags(&B->copied, cudaEventDisableTiming));
     GSRB_CUDA(cudaEventRecord(B->copied, ctx->stream));
@@ -3568,6 +3582,7 @@ gsrb_status_t gsrb_batch_free(gsrb_batch_t B) {
   if (B->ctx) cudaStreamSynchronize(B->ctx->stream);
   if (B->copied) cudaEventDestroy(B->copied);
   if (B->h_desc) cudaFreeHost(B->h_desc);
+  for (BatchDesc* d : B->h_captured) cudaFreeHost(d);
   if (B->d_desc) cudaFree(B->d_desc);
   if (B->d_cta_inst) cudaFree(B->d_cta_inst);
   delete B;

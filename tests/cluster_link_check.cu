@@ -59,7 +59,7 @@ check_kernel(uint32_t steps, int kind, uint32_t bad_rank, uint32_t bad_step, uns
   } while (0)
 
 int main() {
-  constexpr uint32_t n = kClMaxCtas;
+  constexpr uint32_t n = kClCtas;
   uint32_t* d = nullptr;
   CUDA(cudaMalloc(&d, n * kClThreads * sizeof(uint32_t)));
   CUDA(cudaFuncSetAttribute(check_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));

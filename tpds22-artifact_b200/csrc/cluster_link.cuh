@@ -15,11 +15,11 @@
 
 namespace gsrbg {
 
-constexpr uint32_t kClMaxCtas = 16;   // cluster size asked for (8 where 16 cannot be placed)
+constexpr uint32_t kClCtas = 16;      // cluster size
 constexpr uint32_t kClThreads = 512;  // threads per CTA (every warp goes through every step: 1024 cost 0.3 us a step more)
 
 struct ClusterLink {
-  uint4 tab[2][kClMaxCtas];  // the CTAs' records, by parity of the step
+  uint4 tab[2][kClCtas];  // the CTAs' records, by parity of the step
   uint64_t mbar[2];
   uint64_t meet;             // see link_meet
 };
@@ -163,9 +163,8 @@ __device__ __forceinline__ uint32_t link_locate(const ClusterLink& l, uint32_t p
 // again as an even share.  An SM takes about four cycles an edge, so 250 entries
 // of 4 edges on one of 16 CTAs cost 2.0 us beyond the chain; shares drift apart
 // over hundreds of steps only.
-__device__ __forceinline__ bool link_uneven(const LinkSum& s, uint32_t ncta) {
-  static_assert(kClMaxCtas == 16, "shares by shifts");
-  const uint32_t share = (s.x + ncta - 1) >> (ncta == 16 ? 4 : 3);
+__device__ __forceinline__ bool link_uneven(const LinkSum& s) {
+  const uint32_t share = (s.x + kClCtas - 1) / kClCtas;
   return s.max_x > share + share / 2 + 32u;
 }
 

@@ -922,7 +922,7 @@ __global__ void __launch_bounds__(kClThreads, 1) bfs_cluster_kernel(BfsArgs a, u
       }
     }
     auto step = [&](const uint32_t* j, const uint32_t*, uint32_t act) { bfs_cl_push<4>(a, s, L, j, act); };
-    const bool uneven = link_uneven(t, ncta);
+    const bool uneven = link_uneven(t);
     if (uneven) ok = link_meet(s.link, phases, ncta, timeout_ns);
     if (!ok) {
       // gave up: on to the end of the step
@@ -1656,7 +1656,7 @@ __global__ void __launch_bounds__(kClThreads, 1) sssp_cluster_kernel(SsspArgs a,
         };
         walk_group(e.y, e.z - e.y, step);
       };
-      const bool uneven = link_uneven(t, ncta);
+      const bool uneven = link_uneven(t);
       if (uneven) ok = link_meet(s.link, phases, ncta, timeout_ns);
       if (!ok) {
         // gave up: on to the end of the step
@@ -2796,14 +2796,12 @@ size_t with_stage(gsrb_ctx* ctx, const void* fn, int grid, const gsrb_cfg_t& c, 
              : 0;
 }
 
-// CTAs of the cluster that runs thin steps: 16, 8 where 16 cannot be placed,
-// 0 where neither can.
+// CTAs of the cluster that runs thin steps: 0 where it cannot be placed (the grid
+// then runs every step).
 int cluster_ctas(gsrb_ctx* ctx, const void* fn, size_t smem) {
-  for (int k = (int)kClMaxCtas; k >= 8; k /= 2) {
-    int cap = 0;
-    if (coresident_ctas(ctx, fn, (int)kClThreads, smem, k, &cap) == GSRB_OK && cap >= k) return k;
-  }
-  return 0;
+  int cap = 0;
+  const int k = (int)kClCtas;
+  return coresident_ctas(ctx, fn, (int)kClThreads, smem, k, &cap) == GSRB_OK && cap >= k ? k : 0;
 }
 
 // Statistics from a copy of the graph's 32 status words.

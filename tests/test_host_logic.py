@@ -320,6 +320,17 @@ def test_sssp_labels(pol):
     assert y3 == 4.0  # clipped
 
 
+def test_sssp_labels_own_launch(pol):
+    # the width label follows the fastest launch, the library's own among them;
+    # the launch label stays that of the two configurations
+    t = np.array([[9.0, 5.0, 4.0, 4.1, 4.0, 6.0],
+                  [20.0, 10.0, 8.0, 8.0, 8.0, 8.0]])
+    own = np.array([3.0, 2.0, 2.01, 3.0, 4.0, 4.0])
+    y2, y3 = pol.sssp_labels(t, 128.0, own=own)
+    assert abs(y2 - np.mean([np.log2(d / 128.0) for d in (256, 1024)])) < 1e-9 and abs(y3 - np.log2(4.0 / 8.0)) < 1e-9
+    assert pol.sssp_labels(t, 128.0, own=own + 4.0) == pol.sssp_labels(t, 128.0)
+
+
 def test_sssp_features_host(gsrb):
     f = np.zeros(12, np.float32)
     gsrb.lib().gsrb_sssp_features(1 << 20, 16 << 20, 5000, 7, 128.0, 1, 255, 1, f.ctypes.data)

@@ -501,7 +501,10 @@ def train_policy(gsrb, ctx, pol):
                                       "n_m_ms0_ms1": launch}}
 
 
-def bfs_runs(gsrb, ctx, orc, dg, g, params, cfg, reps=3, launch=None, cpu=False):
+def bfs_runs(gsrb, ctx, orc, dg, g, params, cfg, reps=3, launch=None, cpu=False, own_launch=False):
+    """own_launch: the schedules that choose per level run as a user calls them,
+    without a launch configuration (thin levels then run on one cluster); cfg is
+    the plain push arms' then."""
     out = ctx.array(g.nnodes, np.int32)
     t_cpu, want = wall(lambda: orc.bfs(g, 0))
     m_trav = orc.traversed_edges(g, want)
@@ -519,7 +522,8 @@ def bfs_runs(gsrb, ctx, orc, dg, g, params, cfg, reps=3, launch=None, cpu=False)
                        ("heuristic", gsrb.BFS_HEURISTIC), ("learned", gsrb.BFS_LEARNED)):
         ts = []
         for _ in range(reps):
-            rc, st = dg.bfs(0, out, mode, cfg)
+            chooses = mode in (gsrb.BFS_HEURISTIC, gsrb.BFS_LEARNED)
+            rc, st = dg.bfs(0, out, mode, None if own_launch and chooses else cfg)
             gsrb.check(rc, f"bfs {name}")
             ts.append(st.kernel_ms)
         ok = bool(np.array_equal(out.download(), want))
@@ -530,7 +534,7 @@ def bfs_runs(gsrb, ctx, orc, dg, g, params, cfg, reps=3, launch=None, cpu=False)
             res[name]["policy_decisions"] = int(st.decisions)
             res[name]["fallback_level"] = int(st.aux)
             if st.levels <= 64:
-                # per-level schedule (0 push, 1 pull, 2 topology push, 3 one-CTA push)
+                # per-level schedule (0 push, 1 pull, 2 topology push, 3 push on one CTA or cluster)
                 res[name]["dirs"] = [int(x) for x in dg.trace(64)["dir"][: int(st.levels)]]
     res["learned_vs_plain"] = round(res["plain_push"]["ms"] / res["learned"]["ms"], 3)
     if launch is not None:
@@ -636,7 +640,8 @@ def graph_numbers(gsrb, ctx, orc, pol, params, sparams, tune, cache, verify_pr=T
     cache["bfs_rmat"] = best
     res["rmat22"]["launch_tuning"] = _tuning_note(gsrb, best, ttab)
     cfg = tune.cfg_from(best)
-    res["rmat22"]["bfs"] = bfs_runs(gsrb, ctx, orc, dg, rm, params, cfg, launch=pol.launch_candidates(), cpu=True)
+    res["rmat22"]["bfs"] = bfs_runs(gsrb, ctx, orc, dg, rm, params, cfg, launch=pol.launch_candidates(), cpu=True,
+                                     own_launch=True)
     dg.set_sssp_policy(sparams)
     dg.set_launch_choices(*pol.launch_candidates())
     res["rmat22"]["sssp"] = sssp_runs(gsrb, ctx, orc, dg, rm, [("learned", gsrb.SSSP_DELTA_LEARNED, None),
@@ -695,7 +700,7 @@ def graph_numbers(gsrb, ctx, orc, pol, params, sparams, tune, cache, verify_pr=T
     cfg = tune.cfg_from(best)
     res["grid2048"] = {"n": gr.nnodes, "m": gr.nedges, "launch_tuning": _tuning_note(gsrb, best, ttab),
                        "bfs": bfs_runs(gsrb, ctx, orc, dg, gr, params, cfg, reps=2, launch=pol.launch_candidates(),
-                                       cpu=True)}
+                                       cpu=True, own_launch=True)}
     dg.set_sssp_policy(sparams)
     dg.set_launch_choices(*pol.launch_candidates())
     res["grid2048"]["sssp"] = sssp_runs(gsrb, ctx, orc, dg, gr, [("learned", gsrb.SSSP_DELTA_LEARNED, None),

@@ -691,7 +691,7 @@ __device__ __forceinline__ void bfs_run(gsrb::GridSync<V>& bar, bool ok, const B
 // cost 11.4 us at 2 x 512 threads per SM, of which the barrier is two and the
 // rest the chain of trips to L2.  Here a level is: entry (shared memory) ->
 // destinations -> claims with the candidates' row ranges -> shared-memory
-// append -> records exchanged, about 1200 cycles.
+// append -> records exchanged, 2.1 us (about 4200 cycles).
 static_assert(kClEnterFrontier + kClEnterEdges / kClPiece <= kClQueue, "entries and pieces fit one CTA's queue");
 struct BfsClShared {
   uint2 q[2][kClQueue];  // edge ranges of the frontier's vertices, by parity of the level

@@ -1,5 +1,7 @@
-// Persistent barrier-stepped exclusive scan (uint32 with wraparound, and FP32
-// with FP64 offsets).
+// Persistent exclusive scan (uint32 with wraparound, and FP32 with FP64 offsets):
+// a streaming form without a grid barrier for calls without a configuration
+// (scan_stream_kernel, below), and the barrier-stepped forms described here for
+// the others and for arrays that are not 16-byte aligned.
 //
 // Reference: gpu_prescan + sum_scan_blelloch in scan/scan_gsrb.cu:486-804
 // (API scan/scan.h:16-18): 64-element Blelloch tiles (32 threads), a grid
@@ -7,7 +9,7 @@
 // :440-482, :798-799), grid = ceil(N / 64) CTAs that must all be co-resident
 // (N <= 148*32*64 on B200).
 //
-// Here: a fixed co-resident grid (default one 1024-thread CTA per SM) walks the
+// Barrier-stepped: a fixed co-resident grid (default one 1024-thread CTA per SM) walks the
 // input in segments of G chunks (one chunk of `chunk` elements per CTA).  The
 // three phases of the reference run per segment, software-pipelined so that
 // the grid barrier of segment s overlaps the HBM reads of segment s + 1:
@@ -589,9 +591,9 @@ scan_ws_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __restrict
 // one tile ahead, every round waited for the slowest of the CTAs: 3.1 us a round
 // of 32 KiB per SM, 1.5 is the copy).
 //
-// What bounds it: HBM.  2^28 uint32 320 us (1.04 of the measured copy bandwidth),
-// FP32 326 us, where the default call's barrier-stepped form took 657 and 670 us;
-// 3,000,001 FP32 elements 9.1 us for 14.3.
+// What bounds it: HBM.  2^28 uint32 317 us (1.05 of the measured copy bandwidth),
+// FP32 327 us, where the default call's barrier-stepped form took 657 and 670 us;
+// 3,000,001 FP32 elements 8.9 us for 14.3.
 constexpr uint32_t kStreamWarps = 16;  // scanner warps, and slices of a tile
 constexpr uint32_t kSumWarps = 8;
 constexpr uint32_t kStreamThreads = (kStreamWarps + kSumWarps + 2) * 32;

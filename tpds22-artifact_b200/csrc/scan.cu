@@ -592,8 +592,8 @@ scan_ws_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __restrict
 // of 32 KiB per SM, 1.5 is the copy).
 //
 // What bounds it: HBM.  2^28 uint32 317 us (1.05 of the measured copy bandwidth),
-// FP32 327 us, where the default call's barrier-stepped form took 657 and 670 us;
-// 3,000,001 FP32 elements 8.9 us for 14.3.
+// FP32 316 us, where the default call's barrier-stepped form took 657 and 670 us;
+// 3,000,001 FP32 elements 8.5 us for 14.3.
 constexpr uint32_t kStreamWarps = 16;  // scanner warps, and slices of a tile
 constexpr uint32_t kSumWarps = 8;
 constexpr uint32_t kStreamThreads = (kStreamWarps + kSumWarps + 2) * 32;
@@ -746,26 +746,22 @@ scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __rest
       const uint32_t k = i % kStreamStages, q8 = i % kStreamSlots, ph8 = (i / kStreamSlots) & 1u, cnt = tile_cnt(i);
       stream_wait(&full[k], (i / kStreamStages) & 1u, gb, &s_fail);
       Vec x[V];
-      Elem le[V], rt[V];
+      Elem incl[V];  // inclusive prefixes of the lanes' sums, by round of 32 vectors
 #pragma unroll
       for (int r = 0; r < V; ++r) x[r] = load(i, cnt, w * kSlice + 32u * r + lane);
       // (the summers read the stage too, before they publish: the offset waited
       // for below is not there before that)
 #pragma unroll
-      for (int r = 0; r < V; ++r) le[r] = ((x[r].x + x[r].y) + x[r].z) + x[r].w;
-      // (step by step over all rounds: 3,000,001 elements 8.6 us, round by round 8.9)
+      for (int r = 0; r < V; ++r) incl[r] = ((x[r].x + x[r].y) + x[r].z) + x[r].w;
+      // (step by step over all rounds, and the exclusive prefixes only where they
+      // are used: 2^28 FP32 316 us; round by round and ahead of the waits 327)
 #pragma unroll
       for (int o = 1; o < 32; o <<= 1) {
 #pragma unroll
         for (int r = 0; r < V; ++r) {
-          const Elem y = shfl_up(le[r], o);
-          if ((int)lane >= o) le[r] += y;
+          const Elem y = shfl_up(incl[r], o);
+          if ((int)lane >= o) incl[r] += y;
         }
-      }
-#pragma unroll
-      for (int r = 0; r < V; ++r) {
-        rt[r] = shfl_idx(le[r], 31);
-        le[r] = exclusive_of(le[r], ((x[r].x + x[r].y) + x[r].z) + x[r].w);
       }
       stream_wait(&offs[q8], ph8, gb, &s_fail);
       stream_wait(&pref[q8], ph8, gb, &s_fail);
@@ -777,7 +773,7 @@ scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __rest
       for (int r = 0; r < V; ++r) {
         const uint32_t v = w * kSlice + 32u * r + lane;
         const Elem a0 = x[r].x, a1 = a0 + x[r].y, a2 = a1 + x[r].z;
-        const Vec y = out_vec(run + Acc(le[r]), a0, a1, a2);
+        const Vec y = out_vec(run + Acc(exclusive_of(incl[r], a2 + x[r].w)), a0, a1, a2);
         if (4u * v + 3u < cnt) {
           st_hint(reinterpret_cast<Vec*>(dst) + v, y, pol_drop);
         } else {
@@ -786,7 +782,7 @@ scan_stream_kernel(gsrb::GridBarrier gb, const typename ScanT<F32>::Elem* __rest
           for (int q = 0; q < 4; ++q)
             if (4u * v + q < cnt) dst[4u * v + q] = ys[q];
         }
-        run += Acc(rt[r]);
+        run += Acc(shfl_idx(incl[r], 31));
       }
     }
   } else if (w < kStreamWarps + kSumWarps) {
